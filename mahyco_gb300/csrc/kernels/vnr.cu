@@ -877,19 +877,45 @@ struct FaceGrad {
 // remap/UtilesRemap-Impl.h:182-257).  Only cells where the component is not
 // at an extremum need it (the others take "formule 16"): kept out of line so
 // that the slope kernel carries neither its registers nor its code.
+// The face gradients and the limited slope of the component belong to it
+// too: nothing else reads a PenteBorne slope, so components at an extremum
+// (a uniform volume fraction, an absent material) form neither.
 struct PPFluxes {
   double a, b, d;
 };
-__device__ __noinline__ PPFluxes pp_fluxes_call(int plim, double thr, double y0, double yp,
-                                                double ym, double hh, double hp, double hm,
-                                                double grad, double ppa, double ppb, double ppd,
-                                                bool do_ab, bool dual_k) {
-  const PPShape sh = pp_shape(plim, thr, y0, yp, ym, hh, hp, hm, grad);
+struct PPCell {
+  double h0, hp, hm;    // widths: the cell, its "plus" / "minus" neighbours
+  double dxp, dxm;      // centroid distances over the "plus" / "minus" face
+  double ppa, ppb, ppd; // swept lengths: first / second face, dual
+  int lim;              // limiter of the slope and of the reconstruction
+  bool has_gp, has_gm;  // inner faces
+  bool dirx;
+};
+__device__ __noinline__ PPFluxes pp_fluxes_call(const PPCell g, double thr, double y0, double yp,
+                                                double ym, bool do_ab, bool dual_k) {
+  // Remap::computeGradPhiFace{1,2}: (Phi(front) - Phi(back)) / (XcL(front) -
+  // XcL(back)); front / back are the plus / minus neighbours along x, the
+  // minus / plus ones along y
+  const double yf = g.dirx ? yp : ym, yb = g.dirx ? ym : yp;
+  const double gp = g.has_gp ? qdiv(yf - y0, g.dxp) : 0.;
+  const double gm = g.has_gm ? qdiv(y0 - yb, g.dxm) : 0.;
+  const double grad = limit_grad1(g.lim, gp, gm, yp, ym, g.h0, g.hp, g.hm);
+  const PPShape sh = pp_shape(g.lim, thr, y0, yp, ym, g.h0, g.hp, g.hm, grad);
   PPFluxes r;
-  r.a = do_ab ? pp_integral(sh, half(-hh), half(-hh) + ppa, hh, y0, yp, ym, ppa) : 0.;
-  r.b = do_ab ? pp_integral(sh, half(hh) - ppb, half(hh), hh, y0, yp, ym, ppb) : 0.;
-  r.d = dual_k ? pp_integral(sh, 0., ppd, hh, y0, yp, ym, ppd) : 0.;
+  r.a = do_ab ? pp_integral(sh, half(-g.h0), half(-g.h0) + g.ppa, g.h0, y0, yp, ym, g.ppa) : 0.;
+  r.b = do_ab ? pp_integral(sh, half(g.h0) - g.ppb, half(g.h0), g.h0, y0, yp, ym, g.ppb) : 0.;
+  r.d = dual_k ? pp_integral(sh, 0., g.ppd, g.h0, y0, yp, ym, g.ppd) : 0.;
   return r;
+}
+// nonneg((yp - y0) * (ym - y0)): a neighbour with the cell's own bits, all
+// three moderate, makes the product a zero, decided without FP64
+DV bool at_extremum(double y0, double yp, double ym) {
+  constexpr unsigned long long kMod = 2023ull << 52;  // 2^1000
+  const unsigned long long b0 = ubits(y0), bp = ubits(yp), bm = ubits(ym);
+  if ((b0 == bp || b0 == bm) && (b0 & kMag) < kMod && (bp & kMag) < kMod && (bm & kMag) < kMod)
+    return true;
+  asm volatile("");  // keeps the FP64 operations behind the branch
+  return nonneg((yp - y0) * (ym - y0));
 }
 
 // PB: 2 = the run's option decides (batched launches), 0 / 1 = compiled
@@ -937,16 +963,12 @@ struct SweepGradT {
       has_gp = (i > 0);          // bottom face
       has_gm = (i < v.ny - 1);   // top face
     }
-    // With PenteBorne the two face gradients are formed here
-    // (Remap::computeGradPhiFace{1,2}, remap/PhaseRemap1.cc:22-55):
-    // (Phi(front) - Phi(back)) / (XcL(front) - XcL(back)) with the
-    // reference's back / front cells, the "plus" face between c (back) and
-    // cf (front), the "minus" face between cb (back) and c (front).  Each
-    // inner face's gradient is formed by both of its cells with the same
-    // operations, so no face plane is written and read back, and a cell that
-    // takes the no-flux exit below forms neither (the few integrated
-    // components only).  Without PenteBorne FaceGrad formed them once per
-    // face for every component.
+    // With PenteBorne the two face gradients are formed here, by
+    // pp_fluxes_call for the components that need a slope (between the
+    // "plus" face of c and cf and the "minus" face of cb and c): each inner
+    // face's gradient is formed by both of its cells with the same
+    // operations, so no face plane is written and read back.  Without
+    // PenteBorne FaceGrad formed them once per face for every component.
     // Eucclhyd carries momentum (and kinetic energy) after the material
     // components instead of the VNR pseudo-viscosity, and has no dual remap
     const bool euc = (v.scheme == HYDRO_SCHEME_EUCCLHYD);
@@ -1020,15 +1042,10 @@ struct SweepGradT {
     // limited slopes are read; without PenteBorne every slope is stored.
     const int nint = (v.pb_complet == 1) ? (euc ? ncomp : 3 * nb) : (vp ? 2 * nb : nb);
     const int nuse = (cfd && nint < 2 * nb) ? 2 * nb : nint;
-    const int ngrad = (pb == 1) ? nuse : ncomp;
     const int ax = dirx ? 0 : 1;
     const double xc = v.XcL[ax * P + c];
-    // one denominator per face, shared by its components (the IEEE quotient
-    // bit for bit, see shared_div)
     const double dxp = has_gp ? plus_zero(v.XcL[ax * P + cf] - xc) : 1.0;
     const double dxm = has_gm ? plus_zero(xc - v.XcL[ax * P + cb]) : 1.0;
-    const SharedDiv Sp = shared_div(pb == 1 ? dxp : 1.0);
-    const SharedDiv Sm = shared_div(pb == 1 ? dxm : 1.0);
     // Without PenteBorne the order-2 face values (SweepFace) are formed here:
     // a face's value is Phi(cu) + (x_f - XcL(cu)) * slope(cu) of its upwind
     // cell cu = pos(fnv * dxl) ? back : front, with dxl = XcL(front) -
@@ -1069,35 +1086,38 @@ struct SweepGradT {
     const double* Pb = phi_of(v, cb);
     const double* Pp = dirx ? Pf : Pb;  // plus / minus neighbours
     const double* Pm = dirx ? Pb : Pf;
-    double grad[kMaxComp];
-    for (int k = 0; k < ngrad; ++k) {
+    for (int k = 0; pb == 0 && k < ncomp; ++k) {
       const double y0 = Pc[k * P];
       const double yp = Pp[k * P], ym = Pm[k * P];
       double gp = 0., gm = 0.;
-      if (pb == 1) {
-        if (has_gp) gp = qdiv_shared(Sp, Pf[k * P] - y0);
-        if (has_gm) gm = qdiv_shared(Sm, y0 - Pb[k * P]);
-      } else {
-        if (has_gp) gp = v.phiG[k * FP + fp];
-        if (has_gm) gm = v.phiG[k * FP + fm];
-      }
-      grad[k] = limit_grad1(lim, gp, gm, yp, ym, h0, hp, hm);
-      if (pb == 0) {
-        // y0 + s * slope exactly (a zero slope on the integer pipe)
-        if (up_p) v.phiF[k * FP + fp] = addz(y0, mulz(sp, grad[k]));
-        if (up_m) v.phiF[k * FP + fm] = addz(y0, mulz(sm, grad[k]));
-      }
+      if (has_gp) gp = v.phiG[k * FP + fp];
+      if (has_gm) gm = v.phiG[k * FP + fm];
+      const double grad = limit_grad1(lim, gp, gm, yp, ym, h0, hp, hm);
+      // y0 + s * slope exactly (a zero slope on the integer pipe)
+      if (up_p) v.phiF[k * FP + fp] = addz(y0, mulz(sp, grad));
+      if (up_m) v.phiF[k * FP + fm] = addz(y0, mulz(sm, grad));
     }
     if (pb == 1) {
-      const int plim = vp ? v.limiter_pure : v.limiter;
+      PPCell pc;
+      pc.h0 = h0;
+      pc.hp = hp;
+      pc.hm = hm;
+      pc.dxp = dxp;
+      pc.dxm = dxm;
+      pc.ppa = ppa;
+      pc.ppb = ppb;
+      pc.ppd = ppd;
+      pc.lim = lim;
+      pc.has_gp = has_gp;
+      pc.has_gm = has_gm;
+      pc.dirx = dirx;
       double Fr[kMaxComp], Fv[kMaxComp];
-      const double hh = h0;
       for (int k = 0; k < nuse; ++k) {
         const double y0 = Pc[k * P];
         const double yp = Pp[k * P], ym = Pm[k * P];
         const bool dual_k = cfd && k >= nb && k < 2 * nb;
         double fa_, fb_, fd_;
-        if (nonneg((yp - y0) * (ym - y0))) {
+        if (at_extremum(y0, yp, ym)) {
           // "formule 16" (UtilesRemap-Impl.h:201-203): the reference replaces
           // every integral of this component by y0 * swept length, so the
           // reconstruction is not built (y0, a volume fraction here, is
@@ -1106,8 +1126,7 @@ struct SweepGradT {
           fb_ = mul_frac(y0, ppb);
           fd_ = dual_k ? mul_frac(y0, ppd) : 0.;
         } else {
-          const PPFluxes r = pp_fluxes_call(plim, v.threshold, y0, yp, ym, hh, hp, hm, grad[k],
-                                            ppa, ppb, ppd, k < nint, dual_k);
+          const PPFluxes r = pp_fluxes_call(pc, v.threshold, y0, yp, ym, k < nint, dual_k);
           fa_ = r.a;
           fb_ = r.b;
           fd_ = r.d;
