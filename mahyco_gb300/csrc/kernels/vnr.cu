@@ -918,15 +918,195 @@ DV bool at_extremum(double y0, double yp, double ym) {
   return nonneg((yp - y0) * (ym - y0));
 }
 
-// PB: 2 = the run's option decides (batched launches), 0 / 1 = compiled
-// for runs without / with PenteBorne only (plain launches).
-template <int PB>
-struct SweepGradT {
+// One cell of a PenteBorne slope sweep: its neighbours along the sweep
+// (reference naming: cf = "front", right / below; cb = "back", left / above),
+// the reconstruction's inputs, and which components are integrated: volumes
+// always; masses for the pure variant; masses + energies (+ momentum for
+// Eucclhyd) for the "complet" variant (nint); the dual flux needs the mass
+// components (nuse; computeFluxPP, UtilesRemap-Impl.h:259-313).
+struct PBCell {
+  long long c, cf, cb;
+  PPCell pc;
+  double flen;
+  int nint, nuse;
+  bool vp, cfd;
+};
+// Fills X for cell (i, j); false where nothing leaves the cell (put_z(3),
+// the dual flux zero) or outside the mesh.
+template <class PutZ>
+DV bool pb_setup(const RunView& v, int sweep, int i, int j, PBCell& X, const PutZ& put_z) {
+  const Ctrl& C = *v.ctrl;
+  if (i >= v.ny || j >= v.nx) return false;
+  const bool dirx = (sweep == 1) ? C.x_then_y : !C.x_then_y;
+  const long long P = v.pitch;
+  const long long c = (long long)i * v.nx + j;
+  // Eucclhyd carries momentum (and kinetic energy) after the material
+  // components instead of the VNR pseudo-viscosity, and has no dual remap
+  const bool euc = (v.scheme == HYDRO_SCHEME_EUCCLHYD);
+  const bool cfd = !euc && (v.dual_method == 2);
+  const int nb = v.nbmat;
+  const long long n0 = (long long)i * (v.nx + 1) + j;
+  // the four node velocities along the sweep all zeros (and dt finite):
+  // each face velocity is plus_zero(half(+-0 + +-0)) = +0, so every swept
+  // length below is a zero and the cell takes the no-flux exit without
+  // forming them
+  {
+    const long long NP = v.npitch, o = dirx ? 0 : NP;
+    const unsigned long long z = ubits(v.u[o + n0]) | ubits(v.u[o + n0 + 1]) |
+                                 ubits(v.u[o + n0 + v.nx + 1]) | ubits(v.u[o + n0 + v.nx + 2]);
+    if ((z & kMag) == 0 && is_finite(C.dt_n)) {
+      put_z(c, 3);  // both integral planes all +0.0, not stored
+      if (cfd) {
+        const double l = dirx ? ld(v.flv, i) : ld(v.flh, j);
+        const double zf = 0.0 * half(l + l);
+        for (int m = 0; m < nb; ++m) v.DPF[m * P + c] = zf;
+      }
+      return false;
+    }
+  }
+  // the faces' nodes and normals selected by direction, then one set of
+  // operations (two branches, if-converted, would issue both sets): the
+  // left and right faces of an x sweep (fnv_vertical), the bottom and
+  // top faces of a y sweep (fnv_horizontal)
+  const long long W = v.nx + 1;
+  const long long a1 = dirx ? n0 + W : n0 + 1, b0 = dirx ? n0 + 1 : n0 + W;
+  const double fa_v = face_mean(v, dirx, n0, a1);
+  const double fb_v = face_mean(v, dirx, b0, n0 + W + 1);
+  const int qa = dirx ? 0 : 2;
+  const double Fa = mul_pm1(fa_v, nout_at(v, qa, c));
+  const double Fb = mul_pm1(fb_v, nout_at(v, qa + 1, c));
+  const double l = dirx ? ld(v.flv, i) : ld(v.flh, j);
+  X.flen = half(l + l);
+  const double fdual = half(fa_v + fb_v);
+  const double dt = C.dt_n;
+  // Flux_sortant of the two faces and the dual one: the swept lengths
+  X.pc.ppa = half(Fa + fabs(Fa)) * dt;
+  X.pc.ppb = half(Fb + fabs(Fb)) * dt;
+  X.pc.ppd = half(fdual + fabs(fdual)) * dt;
+  // nothing leaves the cell through either face, nor through its dual
+  // half-faces: every flux stored below is then exactly 0 (0 * flen for
+  // the dual one) whatever the slopes, so they are not formed
+  if (iszero(X.pc.ppa) && iszero(X.pc.ppb) && (!cfd || iszero(X.pc.ppd))) {
+    put_z(c, 3);
+    if (cfd) {
+      const double z = 0.0 * X.flen;
+      for (int m = 0; m < nb; ++m) v.DPF[m * P + c] = z;
+    }
+    return false;
+  }
+  long long cf, cb;
+  if (dirx) {
+    cf = (j < v.nx - 1) ? c + 1 : c;
+    cb = (j > 0) ? c - 1 : c;
+    X.pc.has_gp = (j < v.nx - 1);  // right face
+    X.pc.has_gm = (j > 0);         // left face
+  } else {
+    cf = (i > 0) ? c - v.nx : c;
+    cb = (i < v.ny - 1) ? c + v.nx : c;
+    X.pc.has_gp = (i > 0);          // bottom face
+    X.pc.has_gm = (i < v.ny - 1);   // top face
+  }
+  const bool vp = (v.pb_mixte == 1) &&
+                  (v.mixte[c] == 0 && v.mixte[cf] == 0 && v.mixte[cb] == 0 &&
+                   v.pure[c] == v.pure[cf] && v.pure[c] == v.pure[cb]);
+  // "plus" / "minus" neighbours in computeAndLimitGradPhi's argument order
+  const long long cp = dirx ? cf : cb, cm = dirx ? cb : cf;
+  const double* H = dirx ? v.Hx : v.Hy;
+  X.pc.h0 = H[c];
+  X.pc.hp = H[cp];
+  X.pc.hm = H[cm];
+  const int ax = dirx ? 0 : 1;
+  const double xc = v.XcL[ax * P + c];
+  X.pc.dxp = X.pc.has_gp ? plus_zero(v.XcL[ax * P + cf] - xc) : 1.0;
+  X.pc.dxm = X.pc.has_gm ? plus_zero(xc - v.XcL[ax * P + cb]) : 1.0;
+  X.pc.lim = vp ? v.limiter_pure : v.limiter;
+  X.pc.dirx = dirx;
+  X.nint = (v.pb_complet == 1) ? (euc ? v.ncomp : 3 * nb) : (vp ? 2 * nb : nb);
+  X.nuse = (cfd && X.nint < 2 * nb) ? 2 * nb : X.nint;
+  X.c = c;
+  X.cf = cf;
+  X.cb = cb;
+  X.vp = vp;
+  X.cfd = cfd;
+  return true;
+}
+// "formule 16" (UtilesRemap-Impl.h:201-203): at an extremum the reference
+// replaces every integral of the component by y0 * swept length, so the
+// reconstruction is not built (y0, a volume fraction here, is mostly exactly
+// 1 or 0: mul_frac)
+DV PPFluxes pb_extremum(const PPCell& pc, double y0, bool dual_k) {
+  PPFluxes r;
+  r.a = mul_frac(y0, pc.ppa);
+  r.b = mul_frac(y0, pc.ppb);
+  r.d = dual_k ? mul_frac(y0, pc.ppd) : 0.;
+  return r;
+}
+DV void pb_store_dual(const RunView& v, long long c, int m, double d, double ppd, double flen) {
+  if (iszero(ppd)) d = 0.;
+  v.DPF[m * v.pitch + c] = d * flen;
+}
+// The derived fluxes of one side of the cell from its integrals F(k), k <
+// nint (computeFluxPP's end), into out[k * stride].
+template <class FR>
+DV void pb_finish(const RunView& v, const double* Pc, bool vp, const FR& F, double* out,
+                  long long stride) {
+  const long long P = v.pitch;
+  const int nb = v.nbmat, ncomp = v.ncomp;
+  const bool euc = v.scheme == HYDRO_SCHEME_EUCCLHYD;
+  if (v.pb_complet == 1) {
+    double sfm = 0., sfv = plus_zero(F(0));
+    for (int m = 1; m < nb; m++) sfv += F(m);
+    if (dgt(fabs(sfv), v.threshold)) {
+      for (int m = 0; m < nb; m++) {
+        const double f0 = F(m);
+        double f1 = F(nb + m);
+        if (!vp) f1 = div_ip(f1, sfv) * f0;
+        const double f2 = div_ip(F(2 * nb + m), sfv) * f1;
+        sfm = (m == 0) ? plus_zero(f1) : sfm + f1;
+        out[m * stride] = f0;
+        out[(nb + m) * stride] = f1;
+        out[(2 * nb + m) * stride] = f2;
+      }
+      if (euc)
+        for (int k = 3 * nb; k < ncomp; ++k) out[k * stride] = div_ip(F(k), sfv) * sfm;
+      else
+        out[3 * nb * stride] = Pc[3 * nb * P] * sfv;
+    } else {
+      for (int k = 0; k < ncomp; ++k) out[k * stride] = 0.0;
+    }
+  } else {
+    double sfv = 0., sfm = 0.;
+    for (int m = 0; m < nb; m++) {
+      // an absent material's volume flux is exactly 0 (mul_frac)
+      const double f0 = F(m);
+      const double f1 = vp ? F(nb + m) : mul_frac(f0, Pc[(nb + m) * P]);
+      const double f2 = mul_frac(f1, Pc[(2 * nb + m) * P]);
+      sfm = (m == 0) ? plus_zero(f1) : sfm + f1;
+      sfv = (m == 0) ? plus_zero(f0) : sfv + f0;
+      out[m * stride] = f0;
+      out[(nb + m) * stride] = f1;
+      out[(2 * nb + m) * stride] = f2;
+    }
+    if (euc)
+      for (int k = 3 * nb; k < ncomp; ++k) out[k * stride] = Pc[k * P] * sfm;
+    else
+      out[3 * nb * stride] = Pc[3 * nb * P] * sfv;
+  }
+}
+// a zero swept length makes every integral of that side exactly +0.0:
+// recorded in pbz instead of stored (bit 0: dPAr, bit 1: dPAv)
+DV unsigned char pb_zero_sides(const PPCell& pc) {
+  return (iszero(pc.ppa) ? 1 : 0) | (iszero(pc.ppb) ? 2 : 0);
+}
+
+// Slopes and plateau-slope integrals of one cell, by one thread (batched and
+// fused sweeps; a plain launch shares them out in its block, below).
+struct SweepGradPB {
   int sweep;
-  // Fused sweeps (PenteBorne): the cell's flag and integrals go to a tile in
-  // shared memory (tz[ti]; tr / tv[k * ts + ti]) instead of pbz / dPAr /
-  // dPAv, and (phi2) the second sweep reads the Phi of a cell the first
-  // sweep changed from Phi2, where that sweep wrote it.
+  // Fused sweeps: the cell's flag and integrals go to a tile in shared
+  // memory (tz[ti]; tr / tv[k * ts + ti]) instead of pbz / dPAr / dPAv, and
+  // (phi2) the second sweep reads the Phi of a cell the first sweep changed
+  // from Phi2, where that sweep wrote it.
   unsigned char* tz = nullptr;
   double *tr = nullptr, *tv = nullptr;
   int ti = 0, ts = 0;
@@ -934,22 +1114,181 @@ struct SweepGradT {
   DV const double* phi_of(const RunView& v, long long x) const {
     return (phi2 && v.u1s[x] == 0) ? v.Phi2 + x : v.Phi + x;
   }
-  DV void put_z(const RunView& v, long long c, unsigned char z) const {
-    if (tz) tz[ti] = z;
-    else v.pbz[c] = z;
-  }
   __device__ __forceinline__ void operator()(const RunView& v, int i, int j) const {
-    const int pb = (PB == 2) ? v.pb : PB;
-    // no slopes at order 1, nor at order 3 without PenteBorne (batched
-    // launches; the plain cycle does not launch these then)
-    if (v.order <= 1 || (v.order == 3 && pb == 0)) return;
+    PBCell X;
+    auto put_z = [&](long long c, unsigned char z) {
+      if (tz) tz[ti] = z;
+      else v.pbz[c] = z;
+    };
+    if (!pb_setup(v, sweep, i, j, X, put_z)) return;
+    const long long P = v.pitch, c = X.c;
+    const int nb = v.nbmat;
+    const double* Pc = phi_of(v, c);
+    const double* Pf = phi_of(v, X.cf);
+    const double* Pb = phi_of(v, X.cb);
+    const double* Pp = X.pc.dirx ? Pf : Pb;  // plus / minus neighbours
+    const double* Pm = X.pc.dirx ? Pb : Pf;
+    double Fr[kMaxComp], Fv[kMaxComp];
+    for (int k = 0; k < X.nuse; ++k) {
+      const double y0 = Pc[k * P], yp = Pp[k * P], ym = Pm[k * P];
+      const bool dual_k = X.cfd && k >= nb && k < 2 * nb;
+      const PPFluxes r = at_extremum(y0, yp, ym)
+                             ? pb_extremum(X.pc, y0, dual_k)
+                             : pp_fluxes_call(X.pc, v.threshold, y0, yp, ym, k < X.nint, dual_k);
+      if (k < X.nint) {
+        Fr[k] = r.a;
+        Fv[k] = r.b;
+      }
+      if (dual_k) pb_store_dual(v, c, k - nb, r.d, X.pc.ppd, X.flen);
+    }
+    const unsigned char z = pb_zero_sides(X.pc);
+    put_z(c, z);
+    if (!(z & 1)) {
+      auto F = [&](int k) { return Fr[k]; };
+      if (tz) pb_finish(v, Pc, X.vp, F, tr + ti, ts);
+      else pb_finish(v, Pc, X.vp, F, v.dPAr + c, P);
+    }
+    if (!(z & 2)) {
+      auto F = [&](int k) { return Fv[k]; };
+      if (tz) pb_finish(v, Pc, X.vp, F, tv + ti, ts);
+      else pb_finish(v, Pc, X.vp, F, v.dPAv + c, P);
+    }
+  }
+};
+
+// The PenteBorne slopes of a plain launch: a block's (cell, component) pairs
+// that need the reconstruction go to a list in shared memory, from which all
+// of its threads take them in turn.  A reconstruction is about 100 dependent
+// FP64 operations and up to 20 divisions (some 10 us for one thread); a
+// mixed cell has one per material and a cell of a moving pure region one per
+// material it integrates, while its neighbours in the warp have none: by one
+// thread per cell they ran one after another with most lanes idle.
+// rows: rows of 32 cells per block, 1 .. 4; with fewer the block's other
+// threads only work on the list (small meshes, pb_rows).
+constexpr int kPbThreads = kBX * kBY;
+constexpr int kPbParams = 9;  // doubles per cell: the reconstruction's inputs
+inline int pb_max_components(const RunView& v) {
+  const bool euc = v.scheme == HYDRO_SCHEME_EUCCLHYD;
+  if (v.pb_complet == 1) return euc ? v.ncomp : 3 * v.nbmat;
+  return (v.pb_mixte == 1 || (!euc && v.dual_method == 2)) ? 2 * v.nbmat : v.nbmat;
+}
+// integrals of both sides, inputs, list, options and count
+inline size_t pb_smem_bytes(const RunView& v, int rows) {
+  const size_t cells = (size_t)rows * kBX;
+  return cells * ((size_t)(2 * pb_max_components(v) + kPbParams) * sizeof(double) +
+                  (size_t)pb_max_components(v) * sizeof(unsigned short) + 2 * sizeof(int));
+}
+__device__ __forceinline__ void sweep_grad_pb_block(const RunView& v, int sweep, int rows,
+                                                    int ncap) {
+  extern __shared__ double pb_smem[];
+  __shared__ int s_n;
+  const int cells = rows * kBX;
+  double* sa = pb_smem;              // integrals of the dPAr side [k][cell]
+  double* sb = sa + ncap * cells;    // of the dPAv side
+  double* sp = sb + ncap * cells;    // inputs [q][cell]
+  int* so = reinterpret_cast<int*>(sp + kPbParams * cells);
+  int* slim = so + cells;
+  unsigned short* sl = reinterpret_cast<unsigned short*>(slim + cells);
+  const int tid = threadIdx.y * kBX + threadIdx.x;
+  const int i0 = blockIdx.y * rows, j0 = blockIdx.x * kBX;
+  const long long P = v.pitch;
+  const int nb = v.nbmat;
+  PBCell X;
+  bool work = false;
+  if (threadIdx.y < rows)
+    work = pb_setup(v, sweep, i0 + (int)threadIdx.y, j0 + (int)threadIdx.x, X,
+                    [&](long long c, unsigned char z) { v.pbz[c] = z; });
+  if (tid == 0) s_n = 0;
+  if (!__syncthreads_or(work)) return;  // nothing leaves any cell of the block
+  const double *Pc = nullptr, *Pp = nullptr, *Pm = nullptr;
+  if (work) {
+    Pc = v.Phi + X.c;
+    Pp = v.Phi + (X.pc.dirx ? X.cf : X.cb);
+    Pm = v.Phi + (X.pc.dirx ? X.cb : X.cf);
+    bool any = false;
+    for (int k = 0; k < X.nuse; ++k) {
+      const double y0 = Pc[k * P], yp = Pp[k * P], ym = Pm[k * P];
+      const bool dual_k = X.cfd && k >= nb && k < 2 * nb;
+      if (at_extremum(y0, yp, ym)) {
+        const PPFluxes r = pb_extremum(X.pc, y0, dual_k);
+        if (k < X.nint) {
+          sa[k * cells + tid] = r.a;
+          sb[k * cells + tid] = r.b;
+        }
+        if (dual_k) pb_store_dual(v, X.c, k - nb, r.d, X.pc.ppd, X.flen);
+      } else {
+        any = true;
+        sl[atomicAdd(&s_n, 1)] = (unsigned short)(tid | (k << 8));
+      }
+    }
+    if (any) {
+      const PPCell& g = X.pc;
+      const double q[kPbParams] = {g.h0,  g.hp,  g.hm,  g.dxp, g.dxm,
+                                   g.ppa, g.ppb, g.ppd, X.flen};
+#pragma unroll
+      for (int t = 0; t < kPbParams; ++t) sp[t * cells + tid] = q[t];
+      so[tid] = (g.has_gp ? 1 : 0) | (g.has_gm ? 2 : 0) | (X.nint << 2);
+      slim[tid] = g.lim;
+    }
+  }
+  __syncthreads();
+  const int n = s_n;
+  const bool dirx = (sweep == 1) ? v.ctrl->x_then_y : !v.ctrl->x_then_y;
+  const bool cfd = v.scheme != HYDRO_SCHEME_EUCCLHYD && v.dual_method == 2;
+  for (int t = tid; t < n; t += kPbThreads) {
+    const int e = sl[t], w = e & 0xff, k = e >> 8;
+    const int opt = so[w], nint = opt >> 2;
+    PPCell g;
+    g.h0 = sp[w];
+    g.hp = sp[cells + w];
+    g.hm = sp[2 * cells + w];
+    g.dxp = sp[3 * cells + w];
+    g.dxm = sp[4 * cells + w];
+    g.ppa = sp[5 * cells + w];
+    g.ppb = sp[6 * cells + w];
+    g.ppd = sp[7 * cells + w];
+    g.lim = slim[w];
+    g.has_gp = opt & 1;
+    g.has_gm = (opt >> 1) & 1;
+    g.dirx = dirx;
+    const long long c = (long long)(i0 + (w >> 5)) * v.nx + j0 + (w & 31);
+    // the plus / minus neighbours: a face that exists leads to them, the
+    // front one is the plus one along x, the minus one along y
+    const long long st = dirx ? 1 : v.nx;
+    const bool hp = dirx ? g.has_gp : g.has_gm, hm = dirx ? g.has_gm : g.has_gp;
+    const double* Pk = v.Phi + k * P;
+    const bool dual_k = cfd && k >= nb && k < 2 * nb;
+    const PPFluxes r = pp_fluxes_call(g, v.threshold, Pk[c], Pk[hp ? c + st : c],
+                                      Pk[hm ? c - st : c], k < nint, dual_k);
+    if (k < nint) {
+      sa[k * cells + w] = r.a;
+      sb[k * cells + w] = r.b;
+    }
+    if (dual_k) pb_store_dual(v, c, k - nb, r.d, g.ppd, sp[8 * cells + w]);
+  }
+  __syncthreads();
+  if (!work) return;
+  const unsigned char z = pb_zero_sides(X.pc);
+  v.pbz[X.c] = z;
+  if (!(z & 1))
+    pb_finish(v, Pc, X.vp, [&](int k) { return sa[k * cells + tid]; }, v.dPAr + X.c, P);
+  if (!(z & 2))
+    pb_finish(v, Pc, X.vp, [&](int k) { return sb[k * cells + tid]; }, v.dPAv + X.c, P);
+}
+
+// Limited slopes and order-2 face values of runs without PenteBorne.
+struct SweepGradNoPB {
+  int sweep;
+  __device__ __forceinline__ void operator()(const RunView& v, int i, int j) const {
+    // no slopes at order 1, nor at order 3 (batched launches; the plain
+    // cycle does not launch these then)
+    if (v.order != 2) return;
     const Ctrl& C = *v.ctrl;
     if (i >= v.ny || j >= v.nx) return;
     const bool dirx = (sweep == 1) ? C.x_then_y : !C.x_then_y;
-    const long long P = v.pitch;
+    const long long P = v.pitch, FP = v.fpitch;
     const long long c = (long long)i * v.nx + j;
     const double* H = dirx ? v.Hx : v.Hy;
-    // reference naming: cf = "front" (right / below), cb = "back" (left / above)
     long long cf, cb;
     bool has_gp, has_gm;       // gradient faces exist (inner)
     if (dirx) {
@@ -963,90 +1302,16 @@ struct SweepGradT {
       has_gp = (i > 0);          // bottom face
       has_gm = (i < v.ny - 1);   // top face
     }
-    // With PenteBorne the two face gradients are formed here, by
-    // pp_fluxes_call for the components that need a slope (between the
-    // "plus" face of c and cf and the "minus" face of cb and c): each inner
-    // face's gradient is formed by both of its cells with the same
-    // operations, so no face plane is written and read back.  Without
-    // PenteBorne FaceGrad formed them once per face for every component.
-    // Eucclhyd carries momentum (and kinetic energy) after the material
-    // components instead of the VNR pseudo-viscosity, and has no dual remap
-    const bool euc = (v.scheme == HYDRO_SCHEME_EUCCLHYD);
-    const bool cfd = !euc && (v.dual_method == 2);
-    const int ncomp = v.ncomp, nb = v.nbmat;
-    // PenteBorne: Flux_sortant of the two faces, dual normal velocity, face
-    // lengths, and the swept lengths they give
-    double ppa = 0., ppb = 0., ppd = 0., flen = 0.;
-    if (pb == 1) {
-      const long long n0 = (long long)i * (v.nx + 1) + j;
-      // the four node velocities along the sweep all zeros (and dt finite):
-      // each face velocity is plus_zero(half(+-0 + +-0)) = +0, so every
-      // swept length below is a zero and the cell takes the no-flux exit
-      // without forming them
-      {
-        const long long NP = v.npitch, o = dirx ? 0 : NP;
-        const unsigned long long z = ubits(v.u[o + n0]) | ubits(v.u[o + n0 + 1]) |
-                                     ubits(v.u[o + n0 + v.nx + 1]) | ubits(v.u[o + n0 + v.nx + 2]);
-        if ((z & kMag) == 0 && is_finite(C.dt_n)) {
-          put_z(v, c, 3);  // both integral planes all +0.0, not stored
-          if (cfd) {
-            const double l = dirx ? ld(v.flv, i) : ld(v.flh, j);
-            const double zf = 0.0 * half(l + l);
-            for (int m = 0; m < nb; ++m) v.DPF[m * P + c] = zf;
-          }
-          return;
-        }
-      }
-      // the faces' nodes and normals selected by direction, then one set of
-      // operations (two branches, if-converted, would issue both sets): the
-      // left and right faces of an x sweep (fnv_vertical), the bottom and
-      // top faces of a y sweep (fnv_horizontal)
-      const long long W = v.nx + 1;
-      const long long a1 = dirx ? n0 + W : n0 + 1, b0 = dirx ? n0 + 1 : n0 + W;
-      const double fa_v = face_mean(v, dirx, n0, a1);
-      const double fb_v = face_mean(v, dirx, b0, n0 + W + 1);
-      const int qa = dirx ? 0 : 2;
-      const double Fa = mul_pm1(fa_v, nout_at(v, qa, c));
-      const double Fb = mul_pm1(fb_v, nout_at(v, qa + 1, c));
-      const double l = dirx ? ld(v.flv, i) : ld(v.flh, j);
-      flen = half(l + l);
-      const double fdual = half(fa_v + fb_v);
-      const double dt = C.dt_n;
-      ppa = half(Fa + fabs(Fa)) * dt;
-      ppb = half(Fb + fabs(Fb)) * dt;
-      ppd = half(fdual + fabs(fdual)) * dt;
-      // nothing leaves the cell through either face, nor through its dual
-      // half-faces: every flux stored below is then exactly 0 (0 * flen for
-      // the dual one) whatever the slopes, so they are not formed
-      if (iszero(ppa) && iszero(ppb) && (!cfd || iszero(ppd))) {
-        put_z(v, c, 3);
-        if (cfd) {
-          const double z = 0.0 * flen;
-          for (int m = 0; m < nb; ++m) v.DPF[m * P + c] = z;
-        }
-        return;
-      }
-    }
-    const bool vp = (v.pb_mixte == 1) &&
-                    (v.mixte[c] == 0 && v.mixte[cf] == 0 && v.mixte[cb] == 0 &&
-                     v.pure[c] == v.pure[cf] && v.pure[c] == v.pure[cb]);
-    int lim = v.limiter;
-    if ((pb == 1) && vp) lim = v.limiter_pure;
+    const int ncomp = v.ncomp;
+    const int lim = v.limiter;
     // "plus" / "minus" neighbours in computeAndLimitGradPhi's argument order
     const long long cp = dirx ? cf : cb, cm = dirx ? cb : cf;
     const double h0 = H[c], hp = H[cp], hm = H[cm];
-    // which components are integrated with PenteBorne: volumes always;
-    // masses for the pure variant; masses + energies (+ momentum for
-    // Eucclhyd) for the "complet" variant; the dual flux needs the mass
-    // components (computeFluxPP, UtilesRemap-Impl.h:259-313).  Only their
-    // limited slopes are read; without PenteBorne every slope is stored.
-    const int nint = (v.pb_complet == 1) ? (euc ? ncomp : 3 * nb) : (vp ? 2 * nb : nb);
-    const int nuse = (cfd && nint < 2 * nb) ? 2 * nb : nint;
     const int ax = dirx ? 0 : 1;
     const double xc = v.XcL[ax * P + c];
     const double dxp = has_gp ? plus_zero(v.XcL[ax * P + cf] - xc) : 1.0;
     const double dxm = has_gm ? plus_zero(xc - v.XcL[ax * P + cb]) : 1.0;
-    // Without PenteBorne the order-2 face values (SweepFace) are formed here:
+    // The order-2 face values (SweepFace) are formed here:
     // a face's value is Phi(cu) + (x_f - XcL(cu)) * slope(cu) of its upwind
     // cell cu = pos(fnv * dxl) ? back : front, with dxl = XcL(front) -
     // XcL(back), the plus face's denominator above (c its back cell) or the
@@ -1054,10 +1319,7 @@ struct SweepGradT {
     // which writes its value; the slopes themselves are not stored.  (The
     // update cannot form these values: in the first sweep it rewrites Phi,
     // which a neighbour's face value reads.)
-    bool up_p = false, up_m = false;
-    double sp = 0., sm = 0.;
-    long long fp = 0, fm = 0;
-    const long long FP = v.fpitch;
+    long long fp, fm;
     if (dirx) {
       fm = (long long)i * (v.nx + 1) + j;  // left face
       fp = fm + 1;                         // right face
@@ -1065,28 +1327,23 @@ struct SweepGradT {
       fp = (long long)i * v.nx + j;        // bottom face
       fm = fp + v.nx;                      // top face
     }
-    if (pb == 0) {
-      const long long n0 = (long long)i * (v.nx + 1) + j;
-      // x sweep: minus = left face (n0, n0 + W), plus = right face;
-      // y sweep: plus = bottom face (n0, n0 + 1), minus = top face
-      const long long W = v.nx + 1;
-      const long long lo1 = dirx ? n0 + W : n0 + 1, hi0 = dirx ? n0 + 1 : n0 + W;
-      const double f_lo = face_mean(v, dirx, n0, lo1), f_hi = face_mean(v, dirx, hi0, n0 + W + 1);
-      const double fnv_m = dirx ? f_lo : f_hi, fnv_p = dirx ? f_hi : f_lo;
-      const double xf_m = dirx ? ld(v.xs, j) : ld(v.ys, i + 1);
-      const double xf_p = dirx ? ld(v.xs, j + 1) : ld(v.ys, i);
-      up_p = has_gp && pos(fnv_p * dxp);   // c is the plus face's back cell
-      up_m = has_gm && !pos(fnv_m * dxm);  // c is the minus face's front cell
-      sp = plus_zero(xf_p - xc);
-      sm = plus_zero(xf_m - xc);
-    }
-    // Phi of the cell and of its front / back neighbours
-    const double* Pc = phi_of(v, c);
-    const double* Pf = phi_of(v, cf);
-    const double* Pb = phi_of(v, cb);
-    const double* Pp = dirx ? Pf : Pb;  // plus / minus neighbours
-    const double* Pm = dirx ? Pb : Pf;
-    for (int k = 0; pb == 0 && k < ncomp; ++k) {
+    const long long n0 = (long long)i * (v.nx + 1) + j;
+    // x sweep: minus = left face (n0, n0 + W), plus = right face;
+    // y sweep: plus = bottom face (n0, n0 + 1), minus = top face
+    const long long W = v.nx + 1;
+    const long long lo1 = dirx ? n0 + W : n0 + 1, hi0 = dirx ? n0 + 1 : n0 + W;
+    const double f_lo = face_mean(v, dirx, n0, lo1), f_hi = face_mean(v, dirx, hi0, n0 + W + 1);
+    const double fnv_m = dirx ? f_lo : f_hi, fnv_p = dirx ? f_hi : f_lo;
+    const double xf_m = dirx ? ld(v.xs, j) : ld(v.ys, i + 1);
+    const double xf_p = dirx ? ld(v.xs, j + 1) : ld(v.ys, i);
+    const bool up_p = has_gp && pos(fnv_p * dxp);   // c is the plus face's back cell
+    const bool up_m = has_gm && !pos(fnv_m * dxm);  // c is the minus face's front cell
+    const double sp = plus_zero(xf_p - xc);
+    const double sm = plus_zero(xf_m - xc);
+    const double* Pc = v.Phi + c;
+    const double* Pp = v.Phi + cp;
+    const double* Pm = v.Phi + cm;
+    for (int k = 0; k < ncomp; ++k) {
       const double y0 = Pc[k * P];
       const double yp = Pp[k * P], ym = Pm[k * P];
       double gp = 0., gm = 0.;
@@ -1097,96 +1354,15 @@ struct SweepGradT {
       if (up_p) v.phiF[k * FP + fp] = addz(y0, mulz(sp, grad));
       if (up_m) v.phiF[k * FP + fm] = addz(y0, mulz(sm, grad));
     }
-    if (pb == 1) {
-      PPCell pc;
-      pc.h0 = h0;
-      pc.hp = hp;
-      pc.hm = hm;
-      pc.dxp = dxp;
-      pc.dxm = dxm;
-      pc.ppa = ppa;
-      pc.ppb = ppb;
-      pc.ppd = ppd;
-      pc.lim = lim;
-      pc.has_gp = has_gp;
-      pc.has_gm = has_gm;
-      pc.dirx = dirx;
-      double Fr[kMaxComp], Fv[kMaxComp];
-      for (int k = 0; k < nuse; ++k) {
-        const double y0 = Pc[k * P];
-        const double yp = Pp[k * P], ym = Pm[k * P];
-        const bool dual_k = cfd && k >= nb && k < 2 * nb;
-        double fa_, fb_, fd_;
-        if (at_extremum(y0, yp, ym)) {
-          // "formule 16" (UtilesRemap-Impl.h:201-203): the reference replaces
-          // every integral of this component by y0 * swept length, so the
-          // reconstruction is not built (y0, a volume fraction here, is
-          // mostly exactly 1 or 0: mul_frac)
-          fa_ = mul_frac(y0, ppa);
-          fb_ = mul_frac(y0, ppb);
-          fd_ = dual_k ? mul_frac(y0, ppd) : 0.;
-        } else {
-          const PPFluxes r = pp_fluxes_call(pc, v.threshold, y0, yp, ym, k < nint, dual_k);
-          fa_ = r.a;
-          fb_ = r.b;
-          fd_ = r.d;
-        }
-        if (k < nint) {
-          Fr[k] = fa_;
-          Fv[k] = fb_;
-        }
-        if (dual_k) {
-          double d = fd_;
-          if (iszero(ppd)) d = 0.;
-          v.DPF[(k - nb) * P + c] = d * flen;
-        }
-      }
-      // derived fluxes
-      auto finish = [&](double* F, double* out, long long stride) {
-        if (v.pb_complet == 1) {
-          double sfm = 0., sfv = plus_zero(F[0]);
-          for (int m = 1; m < nb; m++) sfv += F[m];
-          if (dgt(fabs(sfv), v.threshold)) {
-            for (int m = 0; m < nb; m++) {
-              if (!vp) F[nb + m] = div_ip(F[nb + m], sfv) * F[m];
-              F[2 * nb + m] = div_ip(F[2 * nb + m], sfv) * F[nb + m];
-              sfm = (m == 0) ? plus_zero(F[nb + m]) : sfm + F[nb + m];
-            }
-            if (euc)
-              for (int k = 3 * nb; k < ncomp; ++k) F[k] = div_ip(F[k], sfv) * sfm;
-            else
-              F[3 * nb] = Pc[3 * nb * P] * sfv;
-          } else {
-            for (int k = 0; k < ncomp; ++k) F[k] = 0.0;
-          }
-        } else {
-          double sfv = 0., sfm = 0.;
-          for (int m = 0; m < nb; m++) {
-            // an absent material's volume flux is exactly 0 (mul_frac)
-            if (!vp) F[nb + m] = mul_frac(F[m], Pc[(nb + m) * P]);
-            F[2 * nb + m] = mul_frac(F[nb + m], Pc[(2 * nb + m) * P]);
-            sfm = (m == 0) ? plus_zero(F[nb + m]) : sfm + F[nb + m];
-            sfv = (m == 0) ? plus_zero(F[m]) : sfv + F[m];
-          }
-          if (euc)
-            for (int k = 3 * nb; k < ncomp; ++k) F[k] = Pc[k * P] * sfm;
-          else
-            F[3 * nb] = Pc[3 * nb * P] * sfv;
-        }
-        for (int k = 0; k < ncomp; ++k) out[k * stride] = F[k];
-      };
-      // a zero swept length makes every integral of that side exactly +0.0:
-      // recorded in pbz instead of stored (bit 0: dPAr, bit 1: dPAv)
-      put_z(v, c, (iszero(ppa) ? 1 : 0) | (iszero(ppb) ? 2 : 0));
-      if (!iszero(ppa)) {
-        if (tz) finish(Fr, tr + ti, ts);
-        else finish(Fr, v.dPAr + c, P);
-      }
-      if (!iszero(ppb)) {
-        if (tz) finish(Fv, tv + ti, ts);
-        else finish(Fv, v.dPAv + c, P);
-      }
-    }
+  }
+};
+
+// Batched launches: each run's own option decides.
+struct SweepGradAny {
+  int sweep;
+  __device__ __forceinline__ void operator()(const RunView& v, int i, int j) const {
+    if (v.pb == 0) SweepGradNoPB{sweep}(v, i, j);
+    else if (v.order > 1) SweepGradPB{sweep}(v, i, j);
   }
 };
 
@@ -2428,10 +2604,14 @@ __global__ void __launch_bounds__(kBX* kBY) k_next_positions(RunView v) { plain_
 __global__ void __launch_bounds__(kBX* kBY) k_face_grad(RunView v, int sweep) { plain_items(v, FaceGrad{sweep}); }
 __global__ void __launch_bounds__(kBX* kBY) k_o3_grad(RunView v, int sweep) { plain_items(v, O3Grad{sweep}); }
 __global__ void __launch_bounds__(kBX* kBY) k_o3_ystar(RunView v, int sweep) { plain_items(v, O3Ystar{sweep}); }
-__global__ void __launch_bounds__(kBX* kBY) k_sweep_grad(RunView v, int sweep) { plain_items(v, SweepGradT<0>{sweep}); }
+__global__ void __launch_bounds__(kBX* kBY) k_sweep_grad(RunView v, int sweep) { plain_items(v, SweepGradNoPB{sweep}); }
 // eight resident blocks: the kernel waits on memory more than it computes
 // at rest; measured faster than the register-limited four to six
-__global__ void __launch_bounds__(kBX* kBY, 8) k_sweep_grad_pb(RunView v, int sweep) { plain_items(v, SweepGradT<1>{sweep}); }
+__global__ void __launch_bounds__(kBX* kBY, 8) k_sweep_grad_pb(RunView v, int sweep, int rows,
+                                                               int ncap) {
+  if (!v.ctrl->active) return;
+  sweep_grad_pb_block(v, sweep, rows, ncap);
+}
 __global__ void __launch_bounds__(kBX* kBY) k_sweep_face(RunView v, int sweep) { plain_items(v, SweepFaceT<2>{sweep}); }
 __global__ void __launch_bounds__(kBX* kBY, 4) k_sweep_face3(RunView v, int sweep) { plain_items(v, SweepFaceT<1>{sweep}); }
 __global__ void __launch_bounds__(kBX* kBY) k_sweep_update(RunView v, int sweep) { plain_items(v, SweepUpdateT<0>{sweep}); }
@@ -2440,7 +2620,7 @@ __global__ void __launch_bounds__(kBX* kBY, 9) k_sweep_update_f(RunView v, int s
 // ------------------------------------------------------- fused remap sweep
 // One launch per sweep for VNR runs with PenteBorne pure at order 2 (the
 // benchmark's options; fused_sweeps_ok): the slopes and plateau-slope
-// integrals of SweepGradT and the update of SweepUpdateT, with the
+// integrals of SweepGradPB and the update of SweepUpdateT, with the
 // integrals and their zero flags kept in shared memory instead of the
 // dPAr / dPAv / pbz planes.  A cell's face values need the integrals of
 // its neighbours along the sweep, so a tile computes them for one cell more
@@ -2493,7 +2673,7 @@ __device__ __forceinline__ void sweep_fused(const RunView& v, int sweep) {
       const int i = by * kFxRows + r;
       if (i >= v.ny) break;  // uniform over the block
       if (j >= 0 && j < v.nx)
-        SweepGradT<1>{sweep, sz, sr, sv, tid, cells, sweep == 2}(v, i, j);
+        SweepGradPB{sweep, sz, sr, sv, tid, cells, sweep == 2}(v, i, j);
       __syncthreads();
       if (tid >= 1 && tid <= kFxCells - 2 && j < v.nx)
         SweepUpdateT<1>{sweep, sz, sr, sv, tid, tid - 1, tid + 1, cells, sweep == 1}(v, i, j);
@@ -2515,7 +2695,7 @@ __device__ __forceinline__ void sweep_fused(const RunView& v, int sweep) {
     for (int s = 0;; ++s) {
       const int g = i0 - 1 + 4 * s + ty;
       if (g >= 0 && g <= i1 && g < v.ny && j < v.nx)
-        SweepGradT<1>{sweep, sz, sr, sv, slot(g), cells, sweep == 2}(v, g, j);
+        SweepGradPB{sweep, sz, sr, sv, slot(g), cells, sweep == 2}(v, g, j);
       __syncthreads();
       const int r = i0 + 4 * (s - 1);
       const int row = r + ty;
@@ -2541,8 +2721,8 @@ __global__ void __launch_bounds__(kBX* kBY, 8) k_final(RunView v) { plain_items(
 __global__ void __launch_bounds__(kBatchThreads, 10) kb_lag_nodes(BatchArgs b) { batch_items(b, LagNodes{}, HYDRO_SCHEME_VNR); }
 __global__ void __launch_bounds__(kBatchThreads, 8) kb_lag_cells(BatchArgs b) { batch_items(b, LagCells{}, HYDRO_SCHEME_VNR); }
 __global__ void __launch_bounds__(kBatchThreads) kb_face_grad(BatchArgs b) { batch_items(b, FaceGrad{b.sweep}); }
-__global__ void __launch_bounds__(kBatchThreads, 8) kb_sweep_grad(BatchArgs b) { batch_items(b, SweepGradT<2>{b.sweep}); }
-__global__ void __launch_bounds__(kBatchThreads, 8) kb_sweep_grad_nopb(BatchArgs b) { batch_items(b, SweepGradT<0>{b.sweep}); }
+__global__ void __launch_bounds__(kBatchThreads, 8) kb_sweep_grad(BatchArgs b) { batch_items(b, SweepGradAny{b.sweep}); }
+__global__ void __launch_bounds__(kBatchThreads, 8) kb_sweep_grad_nopb(BatchArgs b) { batch_items(b, SweepGradNoPB{b.sweep}); }
 __global__ void __launch_bounds__(kBatchThreads) kb_sweep_face(BatchArgs b) { batch_items(b, SweepFaceT<3>{b.sweep}); }
 __global__ void __launch_bounds__(kBatchThreads, 8) kb_sweep_update(BatchArgs b) { batch_items(b, SweepUpdateT<2>{b.sweep}); }
 __global__ void __launch_bounds__(kBatchThreads, 10) kb_dual_grad(BatchArgs b) { batch_items(b, DualGrad{b.sweep}, HYDRO_SCHEME_VNR); }
@@ -2577,6 +2757,14 @@ static dim3 cell_grid(const RunView& v) {
 }
 static dim3 node_grid(const RunView& v) {
   return dim3((v.nx + 1 + kBX - 1) / kBX, (v.ny + 1 + kBY - 1) / kBY);
+}
+
+// Rows of cells per block of the PenteBorne slope kernel: one while blocks of
+// four rows would leave SMs without a block (152 of them), so that a block's
+// list of reconstructions is shared by four times as many threads as cells.
+static int pb_rows(const RunView& v) {
+  const dim3 cg = cell_grid(v);
+  return (long long)cg.x * cg.y <= 152 ? 1 : kBY;
 }
 
 // Computes the node speeds and the initial dt / pressure reductions.
@@ -2626,7 +2814,11 @@ int launch_sweep(const RunView& v, int sweep, cudaStream_t s, const LaunchHook* 
       H(11); k_face_grad<<<fg, blk, 0, s>>>(v, sweep); ++nk;
     }
     H(4);
-    if (v.pb == 1) k_sweep_grad_pb<<<cg, blk, 0, s>>>(v, sweep);
+    if (v.pb == 1) {
+      const int rows = pb_rows(v);
+      k_sweep_grad_pb<<<dim3(cg.x, (v.ny + rows - 1) / rows), blk, pb_smem_bytes(v, rows), s>>>(
+          v, sweep, rows, pb_max_components(v));
+    }
     else k_sweep_grad<<<cg, blk, 0, s>>>(v, sweep);
     ++nk;
   }
