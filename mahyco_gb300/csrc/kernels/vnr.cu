@@ -1370,9 +1370,8 @@ struct SweepGradAny {
 // neighbouring faces: each cell's gradient (eval_grad) enters four faces,
 // each face's interpolated value (eval_ystar) three.  They are computed once
 // per sweep by O3Grad (one thread per cell) and O3Ystar (one thread per
-// inner face) and read by SweepFace for faces whose six-cell stencil is not
-// clamped at the ends of the row / column (the two faces next to each end
-// compute everything themselves).  Same arithmetic, same values.
+// face, the row's / column's end faces included) and read by SweepFace.
+// Same arithmetic, same values.
 // The parabola and its interval (o3_tail) and the face's time-step
 // coefficients behind calls: inline, the compiler issues them under a
 // predicate for every component, also where the face does not move.
@@ -1435,19 +1434,42 @@ struct O3Grad {
                                  o3_value(v, sweep, k, c), o3_value(v, sweep, k, cp));
   }
 };
-// the inner face between positions q-1 and q of cell c's row / column
+// The interpolated value of the face between positions q-1 and q of a row /
+// column, q = 1 .. n-1, and in the boundary faces' slots (q = 0, q = n) the
+// one a clamped stencil has beyond the first / last cell: its two cells and
+// the one outside are the end cell itself, the far one is its neighbour (the
+// other gradients and interpolated values of a clamped stencil are the
+// inner ones: eval_grad clamps like it).  So no face has to form a whole
+// stencil for itself; when the two faces next to each end did, their warps'
+// 39 divisions and per-component work held the face kernel (92 us at 403 x
+// 257 cells, 7 components).
 struct O3Ystar {
   int sweep;
   __device__ __forceinline__ void operator()(const RunView& v, int i, int j) const {
-    if (i >= v.ny || j >= v.nx || !v.o3g) return;
+    if (!v.o3g) return;
     const Ctrl& C = *v.ctrl;
     const bool dirx = (sweep == 1) ? C.x_then_y : !C.x_then_y;
+    if (i >= v.ny + (dirx ? 0 : 1) || j >= v.nx + (dirx ? 1 : 0)) return;
     const long long P = v.pitch, FP = v.fpitch;
-    const long long c = (long long)i * v.nx + j;
     const int q = dirx ? j : i, n = dirx ? v.nx : v.ny;
-    if (q < 1) return;
-    const double* H = dirx ? v.Hx : v.Hy;
     const long long st = dirx ? 1 : v.nx;
+    const double* H = dirx ? v.Hx : v.Hy;
+    const long long f = dirx ? (long long)i * (v.nx + 1) + j : (long long)i * v.nx + j;
+    const long long c = (long long)i * v.nx + j;  // the cell at position q
+    if (q == 0 || q == n) {
+      const long long e = q == 0 ? c : c - st;          // the end cell
+      const long long o = q == 0 ? c + st : c - 2 * st;  // its neighbour (n >= 2)
+      const double he = H[e], ho = H[o];
+      double T[5], G0, A, B;
+      o3_ystar_coef(q == 0 ? he : ho, he, he, q == 0 ? ho : he, T);
+      o3_grad_coef(he, he, he, G0, A, B);
+      for (int k = 0; k < v.ncomp; ++k) {
+        const double y = o3_value(v, sweep, k, e);
+        const double gin = v.o3g[k * P + e], gout = o3_grad(G0, A, B, y, y, y);
+        v.o3y[k * FP + f] = o3_ystar(T, y, y, q == 0 ? gout : gin, q == 0 ? gin : gout);
+      }
+      return;
+    }
     const long long cm = c - st;                           // q-1
     const long long cmm = q > 1 ? cm - st : cm;            // left(q-1)
     const long long cpp = q < n - 1 ? c + st : c;          // right(q)
@@ -1463,7 +1485,6 @@ struct O3Ystar {
     } else {
       o3_ystar_coef(H[cmm], H[cm], H[c], H[cpp], T);
     }
-    const long long f = dirx ? (long long)i * (v.nx + 1) + j : c;
     for (int k = 0; k < v.ncomp; ++k)
       v.o3y[k * FP + f] = o3_ystar(T, o3_value(v, sweep, k, cm), o3_value(v, sweep, k, c),
                                    v.o3g[k * P + cm], v.o3g[k * P + c]);
@@ -1552,17 +1573,17 @@ struct SweepFaceT {
       }
       const double* H = dirx ? v.Hx : v.Hy;
       const double vdt = fnv * C.dt_n;
-      double h[6];
-      for (int t = 0; t < 6; ++t) h[t] = H[cs[t]];
-      // every division of the order-3 value depends on the face only; the
-      // coefficients shared with the neighbouring faces come from O3Coef
-      // unless the stencil is clamped (faces next to the ends)
-      const int q = dirx ? j : i, n = dirx ? v.nx : v.ny;
-      if (v.o3g && q >= 2 && q <= n - 2) {
-        // interior face: gradients and interpolated values from O3Grad /
-        // O3Ystar, only the parabola and its interval here
+      // plain launches: gradients and interpolated values from O3Grad /
+      // O3Ystar (the ends' clamped stencils included), only the parabola and
+      // its interval here; batched launches have neither plane and form the
+      // whole stencil per face (every division depends on the face only)
+      if (ORDERS == 1 || v.o3g) {
+        const double h2 = H[cs[2]], h3 = H[cs[3]];
         O3Dt F;
         bool have_F = false;
+        // |vdt| < 2^500 and widths of at least 2^-500: Q1, Q2 finite
+        const bool qfin = (ubits(vdt) & kMag) < (1523ull << 52) && div_safe_exp(h2) &&
+                          pos(h2) && div_safe_exp(h3) && pos(h3);
         const long long fst = dirx ? 1 : v.nx;  // face stride along the axis
         // A face that does not move: its normal velocity is exactly zero, so
         // (without PenteBorne) the sweep update multiplies its value by a
@@ -1574,8 +1595,8 @@ struct SweepFaceT {
         // overflows).  The value itself is then not formed: 0 is stored
         // (the product's zero may differ in sign, which no later sum sees).
         constexpr unsigned long long kMod = 2023ull << 52;  // 2^1000
-        const bool still = v.pb == 0 && iszero(fnv) && is_finite(C.dt_n) && pos(h[2]) &&
-                           is_finite(h[2]);
+        const bool still = v.pb == 0 && iszero(fnv) && is_finite(C.dt_n) && pos(h2) &&
+                           is_finite(h2);
         for (int k = 0; k < ncomp; ++k) {
           const double ys[3] = {v.o3y[k * FP + fidx - fst], v.o3y[k * FP + fidx],
                                 v.o3y[k * FP + fidx + fst]};
@@ -1588,13 +1609,28 @@ struct SweepFaceT {
             out[k * FP] = 0.0;
             continue;
           }
+          // one value everywhere (an absent material, the fraction of a pure
+          // region): both differences of the parabola are zeros (times the
+          // finite Q1, Q2), its interval is the value (with R1, R2 infinite
+          // too: an undecided comparison keeps the first argument), and the
+          // value itself results (a zero's sign is not seen by any later
+          // sum).  4 of 7 components of a pure two-material cell, 7 of 11 of
+          // a three-material one.
+          const unsigned long long b = ubits(ym);
+          if (qfin && b == ubits(yp) && b == ubits(y1) && b == ubits(y4) && b == ubits(ys[0]) &&
+              b == ubits(ys[1]) && b == ubits(ys[2]) && (b & kMag) < kMod) {
+            out[k * FP] = ym;
+            continue;
+          }
           if (!have_F) {
-            F = o3_dt_call(h[2], h[3], vdt);
+            F = o3_dt_call(h2, h3, vdt);
             have_F = true;
           }
           out[k * FP] = o3_tail_call(F, ys[0], ys[1], ys[2], y1, ym, yp, y4);
         }
       } else {
+        double h[6];
+        for (int t = 0; t < 6; ++t) h[t] = H[cs[t]];
         const O3Face F = o3_face(h, vdt);
         for (int k = 0; k < ncomp; ++k) {
           double y[6];
@@ -2602,8 +2638,12 @@ __global__ void __launch_bounds__(kBX* kBY, 8) k_lag_cells(RunView v) { plain_it
 __global__ void __launch_bounds__(kBX* kBY) k_lag_cells_lo(RunView v) { plain_items(v, LagCellsLagrangeOnly{}); }
 __global__ void __launch_bounds__(kBX* kBY) k_next_positions(RunView v) { plain_items(v, NextPositions{}); }
 __global__ void __launch_bounds__(kBX* kBY) k_face_grad(RunView v, int sweep) { plain_items(v, FaceGrad{sweep}); }
-__global__ void __launch_bounds__(kBX* kBY) k_o3_grad(RunView v, int sweep) { plain_items(v, O3Grad{sweep}); }
-__global__ void __launch_bounds__(kBX* kBY) k_o3_ystar(RunView v, int sweep) { plain_items(v, O3Ystar{sweep}); }
+// Order 3: these wait on memory (eleven components in and out per cell);
+// residency chosen by timing at 1792 x 768 cells, 3 materials: k_o3_grad
+// 86 -> 76 us and k_o3_ystar 122 -> 107 us at twelve blocks against the
+// compiler's eight, k_sweep_face3 179 -> 145 us at seven against five.
+__global__ void __launch_bounds__(kBX* kBY, 12) k_o3_grad(RunView v, int sweep) { plain_items(v, O3Grad{sweep}); }
+__global__ void __launch_bounds__(kBX* kBY, 12) k_o3_ystar(RunView v, int sweep) { plain_items(v, O3Ystar{sweep}); }
 __global__ void __launch_bounds__(kBX* kBY) k_sweep_grad(RunView v, int sweep) { plain_items(v, SweepGradNoPB{sweep}); }
 // eight resident blocks: the kernel waits on memory more than it computes
 // at rest; measured faster than the register-limited four to six
@@ -2613,7 +2653,7 @@ __global__ void __launch_bounds__(kBX* kBY, 8) k_sweep_grad_pb(RunView v, int sw
   sweep_grad_pb_block(v, sweep, rows, ncap);
 }
 __global__ void __launch_bounds__(kBX* kBY) k_sweep_face(RunView v, int sweep) { plain_items(v, SweepFaceT<2>{sweep}); }
-__global__ void __launch_bounds__(kBX* kBY, 4) k_sweep_face3(RunView v, int sweep) { plain_items(v, SweepFaceT<1>{sweep}); }
+__global__ void __launch_bounds__(kBX* kBY, 7) k_sweep_face3(RunView v, int sweep) { plain_items(v, SweepFaceT<1>{sweep}); }
 __global__ void __launch_bounds__(kBX* kBY) k_sweep_update(RunView v, int sweep) { plain_items(v, SweepUpdateT<0>{sweep}); }
 __global__ void __launch_bounds__(kBX* kBY, 9) k_sweep_update_f(RunView v, int sweep) { plain_items(v, SweepUpdateT<1>{sweep}); }
 
@@ -2824,7 +2864,7 @@ int launch_sweep(const RunView& v, int sweep, cudaStream_t s, const LaunchHook* 
   }
   if (v.order == 3) {
     H(16); k_o3_grad<<<cg, blk, 0, s>>>(v, sweep); ++nk;
-    H(17); k_o3_ystar<<<cg, blk, 0, s>>>(v, sweep); ++nk;
+    H(17); k_o3_ystar<<<fg, blk, 0, s>>>(v, sweep); ++nk;
     H(5); k_sweep_face3<<<fg, blk, 0, s>>>(v, sweep); ++nk;
     H(6); k_sweep_update<<<cg, blk, 0, s>>>(v, sweep); ++nk;
   } else if (v.pb == 1) {
