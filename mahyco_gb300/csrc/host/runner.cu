@@ -382,6 +382,7 @@ int place_run(hydro_ctx* ctx, PreparedRun& pr, hydro_run** out, bool wait, bool 
   c0.x_then_y = 1;
   c0.err = 0;
   c0.err_cell = LLONG_MAX;
+  c0.cmat_diag = 1;  // cleared by the set-up where it is not so
   c0.dt_min_bits = 0xFFEFFFFFFFFFFFFFull;  // ordered encoding of +DBL_MAX
   c0.pmax_bits = 0x0010000000000000ull;    // ordered encoding of -DBL_MAX
   r->h_ctrl = c0;

@@ -186,7 +186,8 @@ struct Ctrl {
   unsigned long long pmax_bits;    // ordered encoding of max pressure
   double pmax_prev;                // max pressure of the state at cycle start
   unsigned err;
-  int pad2;
+  int cmat_diag;           // Eucclhyd, set up: every corner matrix has zeros off
+                           // its diagonal (each Cartesian mesh; 0: unknown)
   long long err_cell;
   // output pause (hydro_run_step_to_output): while `pause` is set, a cycle
   // whose start time satisfies the dump condition does not run and `paused`

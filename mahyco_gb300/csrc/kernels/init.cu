@@ -439,7 +439,9 @@ __global__ void __launch_bounds__(kBX* kBY) kd_init_cells_euc(RunView v, int t, 
     lpc[(2 * k) * P + c] = np[0] * lp + nm[0] * lm;
     lpc[(2 * k + 1) * P + c] = np[1] * lp + nm[1] * lm;
     cmat[(3 * k) * P + c] = (np[0] * np[0]) * lp + (nm[0] * nm[0]) * lm;
-    cmat[(3 * k + 1) * P + c] = (np[0] * np[1]) * lp + (nm[0] * nm[1]) * lm;
+    const double m01 = (np[0] * np[1]) * lp + (nm[0] * nm[1]) * lm;
+    cmat[(3 * k + 1) * P + c] = m01;
+    if (!iszero(m01)) atomicAnd(&v.ctrl->cmat_diag, 0);
     cmat[(3 * k + 2) * P + c] = (np[1] * np[1]) * lp + (nm[1] * nm[1]) * lm;
   }
   // initMeshGeometryForCells (Init.cc:106-166): volume, centroid, perimeter
