@@ -831,12 +831,93 @@ struct EucCells {
 
 // --------------------------------------------------------- remap final
 // Eucclhyd::remapCellcenteredVariable (PhaseRemapFinal.cc:17-200)
+//
+// single: a cell that holds one material p (the others' volume, mass and
+// energy +0.0, p's volume and mass positive and finite, the threshold in
+// [0, 1)).  The general path then reduces exactly to volt = vn_p (x + +0 =
+// x), masset = Um_p, vn_p' = vn_p (vol / vn_p) with the others +0, f = mf = 1
+// and +0 (x / x, +0 / x, neither moved by the threshold), rho = 0.0 + Um_p /
+// vn_p', e_p = Ue_p / Um_p + dec, e = 0.0 + e_p, and the others' density +0
+// and energy 0.0 + dec.  A value that leaves these ranges (a negative or NaN
+// density or energy) returns false before any store.  One branch for the
+// cell: 35 -> 8 FP64 instructions, 119 -> 72 us at 1792 x 768 cells and 3
+// materials.
 struct EucFinal {
+  static DV void store_velocity(const RunView& v, long long c, double un0, double un1) {
+    // velocities for the outputs (PhaseRemapFinal.cc:200-213): kept where
+    // the velocity is zero, else pushed away from zero to the threshold
+    const double thr = v.threshold;
+    const long long P = v.pitch;
+    v.uc[c] = un0;
+    v.uc[P + c] = un1;
+    if (pos(un0)) v.uco[c] = smax(un0, thr);
+    else if (neg(un0)) v.uco[c] = smin(un0, -thr);
+    if (pos(un1)) v.uco[P + c] = smax(un1, thr);
+    else if (neg(un1)) v.uco[P + c] = smin(un1, -thr);
+  }
+  static DV bool single(const RunView& v, long long c) {
+    const long long P = v.pitch;
+    const int nb = v.nbmat;
+    const double* U = v.UL + c;
+    const double thr = v.threshold;
+    if (!(nonneg(thr) && dlt(thr, 1.0))) return false;
+    int p = -1, nonzero = 0;
+    double vn = 0., um = 0., ue = 0.;
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      if (m >= nb) break;
+      const double a = U[m * P], b = U[(nb + m) * P], e = U[(2 * nb + m) * P];
+      if ((ubits(a) | ubits(b) | ubits(e)) != 0ull) {
+        p = m;
+        ++nonzero;
+        vn = a;
+        um = b;
+        ue = e;
+      }
+    }
+    // (a warp with a mixed cell takes the general path whole, not both)
+    if (!__all_sync(__activemask(), nonzero == 1)) return false;
+    if (!(pos(vn) && is_finite(vn) && pos(um) && is_finite(um))) return false;
+    const double q0 = U[3 * nb * P], q1 = U[(3 * nb + 1) * P];
+    const double vol = ldg(v.evol, c);
+    const double r = qdiv(vol, vn);
+    if (!(pos(r) && is_finite(r))) return false;
+    const double vnp = mul1z(vn, r);
+    if (!(pos(vnp) && is_finite(vnp))) return false;
+    const double dm = qdiv(um, vnp), pe = qdiv(ue, um);
+    if (neg(dm) || neg(pe) || is_nan(dm) || is_nan(pe)) return false;
+    const double dens = plus_zero(dm);
+    const SharedDiv Smv = shared_div(dens * vol);
+    const double un0 = qdiv_shared(Smv, q0), un1 = qdiv_shared(Smv, q1);
+    double dec = 0.;
+    if (v.conservative == 1)
+      dec = qdiv(U[(3 * nb + 2) * P], um) - 0.5 * (un0 * un0 + un1 * un1);
+    if (!is_finite(dec)) return false;
+    const double em = addz(pe, dec), eo = addz(0.0, dec);
+    const double e = plus_zero(em);
+    if (is_nan(e)) return false;
+    v.mixte[c] = 0;
+    v.pure[c] = p;
+    v.rho[c] = dens;
+    v.e[c] = e;
+    store_velocity(v, c, un0, un1);
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      if (m >= nb) break;
+      const bool here = m == p;
+      v.fm[m * P + c] = here ? 1.0 : 0.0;
+      v.mfm[m * P + c] = here ? 1.0 : 0.0;
+      v.rhom[m * P + c] = here ? dm : 0.0;
+      v.em[m * P + c] = here ? em : eo;
+    }
+    return true;
+  }
   __device__ __forceinline__ void operator()(const RunView& v, int i, int j) const {
     if (i >= v.ny || j >= v.nx) return;
     Ctrl& C = *v.ctrl;
     const long long P = v.pitch;
     const long long c = (long long)i * v.nx + j;
+    if (single(v, c)) return;
     const int nb = v.nbmat;
     const double thr = v.threshold;
     const double* U = v.UL + c;  // second sweep output
@@ -942,15 +1023,8 @@ struct EucFinal {
       atomicMin((unsigned long long*)&C.err_cell, (unsigned long long)c);
     }
     v.rho[c] = dens;
-    v.uc[c] = un0;
-    v.uc[P + c] = un1;
     v.e[c] = e;
-    // velocities for the outputs (PhaseRemapFinal.cc:200-213): kept where
-    // the velocity is zero, else pushed away from zero to the threshold
-    if (pos(un0)) v.uco[c] = smax(un0, thr);
-    else if (neg(un0)) v.uco[c] = smin(un0, -thr);
-    if (pos(un1)) v.uco[P + c] = smax(un1, thr);
-    else if (neg(un1)) v.uco[P + c] = smin(un1, -thr);
+    store_velocity(v, c, un0, un1);
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
       if (m >= nb) break;
@@ -992,7 +1066,7 @@ __global__ void __launch_bounds__(kBX* kBY, 10) ke_final(RunView v) { plain_item
 // Batched launches of the Eucclhyd phases (the batch's VNR runs are skipped;
 // the remap sweeps are the shared batched kernels of vnr.cu).
 constexpr int kE = HYDRO_SCHEME_EUCCLHYD;
-__global__ void __launch_bounds__(kBatchThreads, 12) kbe_cell_pre(BatchArgs b) { batch_items(b, EucCellPre{}, kE); }
+__global__ void __launch_bounds__(kBatchThreads, 8) kbe_cell_pre(BatchArgs b) { batch_items(b, EucCellPre{}, kE); }
 __global__ void __launch_bounds__(kBatchThreads, 8) kbe_nodes(BatchArgs b) { batch_items(b, EucNodes{}, kE); }
 __global__ void __launch_bounds__(kBatchThreads, 8) kbe_cells(BatchArgs b) { batch_items(b, EucCells{}, kE); }
 __global__ void __launch_bounds__(kBatchThreads, 10) kbe_final(BatchArgs b) { batch_items(b, EucFinal{}, kE); }

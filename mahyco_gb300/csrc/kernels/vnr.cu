@@ -2275,20 +2275,20 @@ struct DualUpdate {
 
 // final_cell for a cell that holds one material p: the other materials'
 // volume, mass and energy are +0.0 (bits), p's volume and mass are positive,
-// every material is a perfect gas, the threshold lies in [0, 1), and (for
-// the time step) the four node speeds are +0.0.  The general path then
-// reduces exactly to: volt = vn_p, masset = Um_p (x + +0 = x), rv = vol /
+// every material is a perfect gas and the threshold lies in [0, 1).  The
+// general path then reduces exactly to: volt = vn_p, masset = Um_p (x + +0 = x), rv = vol /
 // vn_p, vn_p' = vn_p * rv and the others +0 * rv = +0 (rv > 0), f = 1 and +0
 // (x / x = 1, +0 / x = +0, neither moved by the threshold), mf likewise,
 // rho = 0.0 + Um_p / vn_p', e = 0.0 + Ue_p / Um_p, p = 0.0 + pm_p with pm_p
 // = (g_p - 1) rho_p e_p, the others' pm = ((g_m - 1) * +0) * +0 (the zero
-// of sign(g_m - 1)), cmassm = cmass and the zero of sign(cmass), and the
-// time-step denominator 0.0 + c.  The few products and quotients that
+// of sign(g_m - 1)), cmassm = cmass and the zero of sign(cmass).  The few products and quotients that
 // remain are the reference's; a value that leaves these ranges (a negative
 // density or energy, a NaN, a non-finite product) returns false before any
 // store, and the general path runs.  One branch for the whole cell: decided
 // per value inside the general path, the shortcuts are if-converted into
-// FP64 instructions that run anyway.
+// FP64 instructions that run anyway.  Moving cells take it like those at
+// rest: FP64 instructions per cell of a moving flow 29 -> 9, 130 -> 74 us at
+// 1001 x 999 cells.
 __device__ __forceinline__ bool final_single(const RunView& v, Ctrl& C, long long c, int nb,
                                              double thr, double vol, const double* vn,
                                              const double* Um, const double* Ue, double Uq,
@@ -2306,9 +2306,8 @@ __device__ __forceinline__ bool final_single(const RunView& v, Ctrl& C, long lon
     }
     ok = ok && eos_of(v, m) == HYDRO_EOS_PERFECT_GAS && is_finite(gm1_of(v, m));
   }
-  if (v.sans_lagrange == 0)
-    ok = ok && (ubits(spd[0]) | ubits(spd[1]) | ubits(spd[2]) | ubits(spd[3])) == 0ull;
-  if (!ok || nonzero != 1) return false;
+  // (a warp with a mixed cell takes the general path whole, not both)
+  if (!__all_sync(__activemask(), ok && nonzero == 1)) return false;
   // p's values by select over the unrolled materials (an index held in a
   // register would put the arrays in local memory)
   double vnp0 = 0., ump = 0., uep = 0.;
@@ -2354,7 +2353,10 @@ __device__ __forceinline__ bool final_single(const RunView& v, Ctrl& C, long lon
     v.pm[m * P + c] = here ? pmp : from_bits(ubits(gm1_of(v, m)) & kS);
   }
   if (v.sans_lagrange == 0) {
-    const double d = div_ip(cflsq, plus_zero(cc));
+    double uc = quarter(spd[0]);
+  #pragma unroll
+    for (int k = 1; k < 4; ++k) uc = addz(uc, quarter(spd[k]));
+    const double d = div_ip(cflsq, addz(uc, cc));
     if (!is_nan(d)) dtb = ord_bits(d) < dtb ? ord_bits(d) : dtb;
   }
   if (!is_nan(pres)) pb = ord_bits(pres) > pb ? ord_bits(pres) : pb;
