@@ -296,7 +296,7 @@ int capture_graph(BatchPlan* p, int cycles) {
   cudaGraph_t g;
   CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   int nk = 0;
-  for (int k = 0; k < cycles; ++k) nk = launch_batch_cycle(p->L, s, nullptr);
+  for (int k = 0; k < cycles; ++k) nk = launch_batch_cycle(p->L, s, nullptr, &p->ctx->fork);
   cudaError_t e = cudaStreamEndCapture(s, &g);
   if (e != cudaSuccess)
     return fail(-40, std::string("batch graph capture: ") + cudaGetErrorString(e));

@@ -182,6 +182,13 @@ int validate(const hydro_spec& s) {
   return 0;
 }
 
+void destroy_fork(CycleFork& f) {
+  for (auto& ev : f.ev)
+    if (ev) cudaEventDestroy((cudaEvent_t)ev);
+  if (f.side) cudaStreamDestroy((cudaStream_t)f.side);
+  f = CycleFork{};
+}
+
 }  // namespace
 
 extern "C" {
@@ -204,9 +211,24 @@ int hydro_ctx_create(int device, size_t budget, hydro_ctx** out) {
     delete c;
     return fail(-3, std::string("cudaStreamCreate: ") + cudaGetErrorString(e));
   }
+  cudaStream_t side = nullptr;
+  e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
+  c->fork.side = side;
+  for (auto& ev : c->fork.ev) {
+    cudaEvent_t x = nullptr;
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&x, cudaEventDisableTiming);
+    ev = x;
+  }
+  if (e != cudaSuccess) {
+    destroy_fork(c->fork);
+    cudaStreamDestroy(c->stream);
+    delete c;
+    return fail(-3, std::string("cudaStreamCreate: ") + cudaGetErrorString(e));
+  }
   // the pinned staging and host copy threads of hydro_run_fetch, set up
   // with the context rather than inside a run's first fetch
   if (int rc = create_fetch_stage(c->num_sms, &c->fetch)) {
+    destroy_fork(c->fork);
     cudaStreamDestroy(c->stream);
     delete c;
     return rc;
@@ -225,6 +247,7 @@ void hydro_ctx_destroy(hydro_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   destroy_fetch_stage(c->fetch);
   c->fetch = nullptr;
+  destroy_fork(c->fork);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
 }
@@ -451,7 +474,7 @@ int build_graph(hydro_run* r, int cycles) {
   cudaGraph_t g;
   CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   int nk = 0;
-  for (int k = 0; k < cycles; ++k) nk = launch_cycle(r->v, s, nullptr);
+  for (int k = 0; k < cycles; ++k) nk = launch_cycle(r->v, s, nullptr, &r->ctx->fork);
   cudaError_t e = cudaStreamEndCapture(s, &g);
   if (e != cudaSuccess) return fail(-40, std::string("graph capture: ") + cudaGetErrorString(e));
   e = cudaGraphInstantiate(&r->graph, g, 0);

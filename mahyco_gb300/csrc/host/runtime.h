@@ -16,10 +16,12 @@ namespace hydro {
 
 void launch_prologue(const RunView& v, cudaStream_t s);
 int launch_device_init(const RunView& v, int test_case, int init_variant, cudaStream_t s);
-int launch_cycle(const RunView& v, cudaStream_t s, const LaunchHook* hook);
+int launch_cycle(const RunView& v, cudaStream_t s, const LaunchHook* hook,
+                 const CycleFork* fork = nullptr);
 void launch_node_mass(const RunView& v, cudaStream_t s);
 int launch_euc_out_pressure(const RunView& v, double* out, cudaStream_t s);
-int launch_batch_cycle(const BatchLaunch& L, cudaStream_t s, const LaunchHook* hook);
+int launch_batch_cycle(const BatchLaunch& L, cudaStream_t s, const LaunchHook* hook,
+                       const CycleFork* fork = nullptr);
 int batch_occupancy(int* blocks_per_sm, int variant);
 int measure_fp64_peak(int device, double* tflops);
 
@@ -64,6 +66,7 @@ struct hydro_ctx {
   size_t budget = 0;       // bytes of run state the context may hold (0: no cap)
   size_t used = 0;         // bytes of run state held
   cudaStream_t stream = nullptr;
+  hydro::CycleFork fork;   // second stream and events of captured cycles
   std::mutex mu;
   hydro::BatchPlan* plan = nullptr;   // batch engine (lazily created)
   hydro::ServeState* serve = nullptr; // serving loop (lazily created)

@@ -219,6 +219,13 @@ __device__ __forceinline__ bool output_pause_here(Ctrl& C) {
 }
 #endif
 
+// A second stream on which a captured cycle's independent launches run beside
+// the others (fork and join by events); null: all in order on one stream.
+struct CycleFork {
+  void* side = nullptr;      // cudaStream_t
+  void* ev[4] = {};          // cudaEvent_t
+};
+
 // Per-kernel timing hook for launch_cycle.
 using LaunchHook = std::function<void(int)>;
 constexpr int kNumKernelKinds = 20;

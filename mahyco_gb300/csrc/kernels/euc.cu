@@ -30,7 +30,8 @@
 
 namespace hydro {
 
-int launch_sweep(const RunView& v, int sweep, cudaStream_t s, const LaunchHook* hook);
+int launch_sweep(const RunView& v, int sweep, cudaStream_t s, const LaunchHook* hook,
+                 const std::function<void(int)>& before);
 
 namespace {
 
@@ -1139,7 +1140,7 @@ int launch_cycle_euc(const RunView& v, cudaStream_t s, const LaunchHook* hook) {
   H(12); ke_cell_pre<<<cg, blk, 0, s>>>(v); ++nk;
   H(13); ke_nodes<<<ng, blk, 0, s>>>(v); ++nk;
   H(14); ke_cells<<<cg, blk, 0, s>>>(v); ++nk;
-  for (int sweep = 1; sweep <= 2; ++sweep) nk += launch_sweep(v, sweep, s, hook);
+  for (int sweep = 1; sweep <= 2; ++sweep) nk += launch_sweep(v, sweep, s, hook, nullptr);
   H(15); ke_final<<<cg, blk, 0, s>>>(v); ++nk;
   H(10); ke_end<<<1, 1, 0, s>>>(v); ++nk;
   H(-1);

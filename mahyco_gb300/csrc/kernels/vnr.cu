@@ -2,7 +2,8 @@
 //
 // Cycle structure (reference: Vnr::executeTimeLoopN, vnr_remap/VnrRemap.cc
 // :127-222):
-//   k_begin        dt_{n+1}, t_{n+1} from the previous cycle's reductions
+//   k_begin        dt_{n+1}, t_{n+1} from the previous cycle's reductions, which it
+//                  resets
 //   k_lag_nodes    node mass, node velocity + boundary conditions, Lagrange
 //                  node positions                       (PhaseLagrange.cc,
 //                                                        ConditionsLimites.cc)
@@ -124,8 +125,10 @@ __device__ __forceinline__ void end_at(const RunView& v) {
   if (C.err & ~HYDRO_ERR_NEGATIVE) C.done = 1;
 }
 
-__global__ void k_begin(RunView v) { begin_at(v); }
-__global__ void k_reset_reductions(RunView v) { reset_at(v); }
+__global__ void k_begin(RunView v) {
+  begin_at(v);
+  reset_at(v);
+}
 __global__ void k_end(RunView v) { end_at(v); }
 
 // block-wide min / max of ordered encodings, one atomic per block
@@ -155,9 +158,11 @@ __device__ void block_reduce_minmax(unsigned long long dtv,
       dtv = a < dtv ? a : dtv;
       pv = b > pv ? b : pv;
     }
+    // (the slots only fall / rise: a block that cannot change them leaves
+    // them alone)
     if (lane == 0) {
-      atomicMin(&C->dt_min_bits, dtv);
-      atomicMax(&C->pmax_bits, pv);
+      if (dtv < __ldcg(&C->dt_min_bits)) atomicMin(&C->dt_min_bits, dtv);
+      if (pv > __ldcg(&C->pmax_bits)) atomicMax(&C->pmax_bits, pv);
     }
   }
   // the shared slots are reused by the next tile of a batched block
@@ -2833,14 +2838,19 @@ const char* const kKernelNames[kNumKernelKinds] = {
 // One directional remap sweep (Remap::computeGradPhiFace, computeGradPhi,
 // computeUpwindFaceQuantitiesForProjection, computeUremap) on stream s,
 // shared by both Lagrange schemes.  Returns the number of kernels.
-int launch_sweep(const RunView& v, int sweep, cudaStream_t s, const LaunchHook* hook) {
+// before(stage), stage 0 ahead of the slopes, 1 ahead of the update: where a
+// forked cycle joins.
+int launch_sweep(const RunView& v, int sweep, cudaStream_t s, const LaunchHook* hook,
+                 const std::function<void(int)>& before) {
   const dim3 blk(kBX, kBY);
   const dim3 cg = cell_grid(v), fg = node_grid(v);
   int nk = 0;
   auto H = [&](int kind) {
     if (hook) (*hook)(kind);
   };
+  if (before) before(0);
   if (v.Phi2) {
+    if (before) before(1);
     // one kernel per direction; the one whose direction this sweep is not
     // returns at once (the direction is decided on the device)
     H(19);
@@ -2868,9 +2878,11 @@ int launch_sweep(const RunView& v, int sweep, cudaStream_t s, const LaunchHook* 
     H(16); k_o3_grad<<<cg, blk, 0, s>>>(v, sweep); ++nk;
     H(17); k_o3_ystar<<<fg, blk, 0, s>>>(v, sweep); ++nk;
     H(5); k_sweep_face3<<<fg, blk, 0, s>>>(v, sweep); ++nk;
+    if (before) before(1);
     H(6); k_sweep_update<<<cg, blk, 0, s>>>(v, sweep); ++nk;
   } else if (v.pb == 1) {
     // PenteBorne, orders 1-2: the update forms its face values
+    if (before) before(1);
     H(6); k_sweep_update_f<<<cg, blk, 0, s>>>(v, sweep); ++nk;
   } else {
     // without PenteBorne the slope kernel wrote the order-2 face values; at
@@ -2878,6 +2890,7 @@ int launch_sweep(const RunView& v, int sweep, cudaStream_t s, const LaunchHook* 
     if (v.order == 1) {
       H(5); k_sweep_face<<<fg, blk, 0, s>>>(v, sweep); ++nk;
     }
+    if (before) before(1);
     H(6); k_sweep_update<<<cg, blk, 0, s>>>(v, sweep); ++nk;
   }
   return nk;
@@ -2885,7 +2898,25 @@ int launch_sweep(const RunView& v, int sweep, cudaStream_t s, const LaunchHook* 
 
 int launch_cycle_euc(const RunView& v, cudaStream_t s, const LaunchHook* hook);
 
-int launch_cycle(const RunView& v, cudaStream_t s, const LaunchHook* hook) {
+// The dual remap's launches that the cell sweeps do not need run on the
+// fork's second stream, when there is one (a captured cycle):
+//   dual_grad 1 (velocities, Lagrange positions)  beside the Lagrange cells
+//                                                 and the first sweep
+//   dual_update 1, dual_grad 2                    beside the second sweep
+// Joins: dual_update 1 after update 1 (its mass-flux shares); update 2, which
+// writes the shares anew, after dual_update 1 (PenteBorne's dual flux: the
+// slopes 2 write them); dual_update 2 after dual_grad 2 and update 2 (which
+// reads the velocities it changes).  A 200 x 10 deck's cycle has twelve
+// launches in a row instead of fifteen: 97 -> 78 us a cycle; 2048 x 2048 cells
+// at rest 1106 -> 1099 us.  (Folding the start and end of the cycle into the first
+// and last kernels, by a ticket per block, gained nothing more: 78 us.)
+static void fork_wait(cudaStream_t to, cudaStream_t from, void* ev) {
+  cudaEventRecord((cudaEvent_t)ev, from);
+  cudaStreamWaitEvent(to, (cudaEvent_t)ev, 0);
+}
+
+int launch_cycle(const RunView& v, cudaStream_t s, const LaunchHook* hook,
+                 const CycleFork* fork) {
   if (v.scheme == HYDRO_SCHEME_EUCCLHYD) return launch_cycle_euc(v, s, hook);
   const dim3 blk(kBX, kBY);
   const dim3 cg = cell_grid(v), ng = node_grid(v);
@@ -2894,7 +2925,6 @@ int launch_cycle(const RunView& v, cudaStream_t s, const LaunchHook* hook) {
     if (hook) (*hook)(kind);
   };
   H(0); k_begin<<<1, 1, 0, s>>>(v); ++nk;
-  H(1); k_reset_reductions<<<1, 1, 0, s>>>(v); ++nk;
   H(2); k_lag_nodes<<<ng, blk, 0, s>>>(v); ++nk;
   if (v.projection == 0) {
     // the Lagrange phase only: its cell kernel reduces the next dt, and the
@@ -2905,12 +2935,33 @@ int launch_cycle(const RunView& v, cudaStream_t s, const LaunchHook* hook) {
     H(-1);
     return nk;
   }
-  H(3); k_lag_cells<<<cg, blk, 0, s>>>(v); ++nk;
-  for (int sweep = 1; sweep <= 2; ++sweep) {
-    nk += launch_sweep(v, sweep, s, hook);
-    H(7); k_dual_grad<<<ng, blk, 0, s>>>(v, sweep); ++nk;
-    H(8); k_dual_update<<<ng, blk, 0, s>>>(v, sweep); ++nk;
+  cudaStream_t d = fork ? (cudaStream_t)fork->side : s;
+  if (fork) {
+    fork_wait(d, s, fork->ev[0]);
+    k_dual_grad<<<ng, blk, 0, d>>>(v, 1); ++nk;
   }
+  H(3); k_lag_cells<<<cg, blk, 0, s>>>(v); ++nk;
+  nk += launch_sweep(v, 1, s, hook, nullptr);
+  if (!fork) {
+    H(7); k_dual_grad<<<ng, blk, 0, s>>>(v, 1); ++nk;
+  } else {
+    fork_wait(d, s, fork->ev[1]);
+  }
+  H(8); k_dual_update<<<ng, blk, 0, d>>>(v, 1); ++nk;
+  if (fork) {
+    cudaEventRecord((cudaEvent_t)fork->ev[2], d);
+    k_dual_grad<<<ng, blk, 0, d>>>(v, 2); ++nk;
+  }
+  const int join = v.dual_method == 2 ? 0 : 1;
+  nk += launch_sweep(v, 2, s, hook, [&](int stage) {
+    if (fork && stage == join) cudaStreamWaitEvent(s, (cudaEvent_t)fork->ev[2], 0);
+  });
+  if (!fork) {
+    H(7); k_dual_grad<<<ng, blk, 0, s>>>(v, 2); ++nk;
+  } else {
+    fork_wait(s, d, fork->ev[3]);
+  }
+  H(8); k_dual_update<<<ng, blk, 0, s>>>(v, 2); ++nk;
   H(9); k_final<<<cg, blk, 0, s>>>(v); ++nk;
   H(10); k_end<<<1, 1, 0, s>>>(v); ++nk;
   H(-1);
@@ -2928,8 +2979,11 @@ int batch_occupancy_euc(int* blocks_per_sm);
 // over its own runs (their phase kernels skip the other scheme's tiles,
 // and are launched only when the batch holds runs of that scheme), the
 // remap sweeps over all.
+// (fork: the dual remap's independent launches on a second stream, as in
+// launch_cycle; the slopes of a batch with PenteBorne may write a dual flux,
+// so they wait for dual_update 1.)
 int launch_batch_cycle(const BatchLaunch& L, cudaStream_t s,
-                       const LaunchHook* hook) {
+                       const LaunchHook* hook, const CycleFork* fork) {
   int nk = 0;
   auto H = [&](int kind) {
     if (hook) (*hook)(kind);
@@ -2957,11 +3011,23 @@ int launch_batch_cycle(const BatchLaunch& L, cudaStream_t s,
     H(2); kb_lag_nodes<<<L.grid[kPhLagNodes], T, 0, s>>>(args(kPhLagNodes, 0)); ++nk;
   }
   if (L.any_euc) euc(13, kPhEucNodes);
+  if (L.any_vnr && fork) {
+    fork_wait((cudaStream_t)fork->side, s, fork->ev[0]);
+    kb_dual_grad<<<L.grid[kPhDualGrad], T, 0, (cudaStream_t)fork->side>>>(args(kPhDualGrad, 1));
+    ++nk;
+  }
   if (L.any_vnr) {
     H(3); kb_lag_cells<<<L.grid[kPhLagCells], T, 0, s>>>(args(kPhLagCells, 0)); ++nk;
   }
   if (L.any_euc) euc(14, kPhEucCells);
+  if (!L.any_vnr) fork = nullptr;
+  cudaStream_t d = fork ? (cudaStream_t)fork->side : s;
+  auto dual_grad = [&](int sweep) {
+    H(7); kb_dual_grad<<<L.grid[kPhDualGrad], T, 0, d>>>(args(kPhDualGrad, sweep)); ++nk;
+  };
   for (int sweep = 1; sweep <= 2; ++sweep) {
+    if (fork && sweep == 2 && !(L.variant & kBatchNoPB))
+      cudaStreamWaitEvent(s, (cudaEvent_t)fork->ev[2], 0);
     if (L.any_order2) {
       if (L.any_face_grad) {
         H(11); kb_face_grad<<<L.grid[kPhFaceGrad], T, 0, s>>>(args(kPhFaceGrad, sweep)); ++nk;
@@ -2979,10 +3045,23 @@ int launch_batch_cycle(const BatchLaunch& L, cudaStream_t s,
     if (L.any_face) {
       H(5); kb_sweep_face<<<L.grid[kPhSweepFace], T, 0, s>>>(args(kPhSweepFace, sweep)); ++nk;
     }
+    if (fork && sweep == 2 && (L.variant & kBatchNoPB))
+      cudaStreamWaitEvent(s, (cudaEvent_t)fork->ev[2], 0);
     H(6); kb_sweep_update<<<L.grid[kPhSweepUpdate], T, 0, s>>>(args(kPhSweepUpdate, sweep)); ++nk;
-    if (L.any_vnr) {
-      H(7); kb_dual_grad<<<L.grid[kPhDualGrad], T, 0, s>>>(args(kPhDualGrad, sweep)); ++nk;
-      H(8); kb_dual_update<<<L.grid[kPhDualUpdate], T, 0, s>>>(args(kPhDualUpdate, sweep)); ++nk;
+    if (!L.any_vnr) continue;
+    if (!fork) {
+      dual_grad(sweep);
+    } else if (sweep == 1) {
+      fork_wait(d, s, fork->ev[1]);
+    } else {
+      fork_wait(s, d, fork->ev[3]);
+    }
+    H(8);
+    kb_dual_update<<<L.grid[kPhDualUpdate], T, 0, sweep == 1 ? d : s>>>(args(kPhDualUpdate, sweep));
+    ++nk;
+    if (fork && sweep == 1) {
+      cudaEventRecord((cudaEvent_t)fork->ev[2], d);
+      dual_grad(2);
     }
   }
   if (L.any_vnr) {
