@@ -423,27 +423,37 @@ HD void lpc_npc(const double* xp, const double* xpp, const double* xpm, double o
   out[1] = na1 * la + nb1 * lb;
 }
 
+// With S_k = X_k + X_kp (the sum of side k's two nodes) and M_k = S_k / 2, the
+// four cross products of a corner k are, in the reference's order, centre x
+// M_km, M_km x X_k, X_k x M_k and M_k x centre: the first is the exact negative
+// of the last one of corner km (the same two products subtracted the other
+// way round; a zero's sign is not seen: the volume's sum starts from +0), and
+// S_k serves the middles and the centroid.  About 100 FP64 operations instead of
+// 132, in the kernel that carries most of them.
 HD CellGeom vnr_cell_geometry(const double X[4][2], bool widths) {
   CellGeom G;
-  double xc0 = plus_zero(X[0][0]), xc1 = plus_zero(X[0][1]);
+  double S[4][2], Mx[4], My[4];
 #pragma unroll
-  for (int k = 1; k < 4; ++k) {
-    xc0 = xc0 + X[k][0];
-    xc1 = xc1 + X[k][1];
+  for (int k = 0; k < 4; ++k) {
+    const int kp = (k + 1) & 3;
+    S[k][0] = X[k][0] + X[kp][0];
+    S[k][1] = X[k][1] + X[kp][1];
+    Mx[k] = half(S[k][0]);
+    My[k] = half(S[k][1]);
   }
-  xc0 = quarter(xc0);
-  xc1 = quarter(xc1);
+  // ((0.0 + X_0) + X_1) + ..: 0.0 + (X_0 + X_1), which is -0 only when both are
+  const double xc0 = quarter((plus_zero(S[0][0]) + X[2][0]) + X[3][0]);
+  const double xc1 = quarter((plus_zero(S[0][1]) + X[2][1]) + X[3][1]);
+  double c41[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) c41[k] = Mx[k] * xc1 - My[k] * xc0;
   double vol = 0.0;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    const int km = (k + 3) & 3, kp = (k + 1) & 3;
-    const double x2a = half(X[km][0] + X[k][0]), x2b = half(X[km][1] + X[k][1]);
-    const double x4a = half(X[kp][0] + X[k][0]), x4b = half(X[kp][1] + X[k][1]);
-    const double c12 = xc0 * x2b - xc1 * x2a;
-    const double c23 = x2a * X[k][1] - x2b * X[k][0];
-    const double c34 = X[k][0] * x4b - X[k][1] * x4a;
-    const double c41 = x4a * xc1 - x4b * xc0;
-    const double t = half(c12 + c23 + c34 + c41);
+    const int km = (k + 3) & 3;
+    const double c23 = Mx[km] * X[k][1] - My[km] * X[k][0];
+    const double c34 = X[k][0] * My[k] - X[k][1] * Mx[k];
+    const double t = half(((c23 - c41[km]) + c34) + c41[k]);
     vol = (k == 0) ? plus_zero(t) : vol + t;
   }
   G.vol = vol;
@@ -452,7 +462,7 @@ HD CellGeom vnr_cell_geometry(const double X[4][2], bool widths) {
   for (int k = 0; k < 4; ++k) {
     const int kp = (k + 1) & 3;
     const double cr = X[k][0] * X[kp][1] - X[k][1] * X[kp][0];
-    const double t0 = cr * (X[k][0] + X[kp][0]), t1 = cr * (X[k][1] + X[kp][1]);
+    const double t0 = cr * S[k][0], t1 = cr * S[k][1];
     r0 = (k == 0) ? plus_zero(t0) : r0 + t0;
     r1 = (k == 0) ? plus_zero(t1) : r1 + t1;
   }
