@@ -265,10 +265,14 @@ HD double div_shared(const SharedDiv& S, double a) {
 // sum is the single square, and sqrt(RN(x*x)) = |x| for binary floating
 // point with correct rounding whenever x*x neither overflows nor
 // underflows (exponents within [-500, 500] here; checked on 2e8 values).
+// The same holds for a component 2^28 times smaller (by exponents): its
+// square is below half an ulp of the other's rounded square, which the sum
+// then rounds to (a face tilted by rounding noise, a flow along one axis).
 HD double face_len(double a, double b) {
   if (iszero(a) && iszero(b)) return 0.0;  // sqrt(+0)
-  if (iszero(b) && div_safe_exp(a)) return fabs(a);
-  if (iszero(a) && div_safe_exp(b)) return fabs(b);
+  const int ea = (int)((ubits(a) >> 52) & 0x7ffu), eb = (int)((ubits(b) >> 52) & 0x7ffu);
+  if (eb <= ea - 28 && div_safe_exp(a)) return fabs(a);
+  if (ea <= eb - 28 && div_safe_exp(b)) return fabs(b);
   double r = mul_ip(a, a);  // 0.0 + a square (never -0) is the square
   r = add_ip(r, mul_ip(b, b));
   return sqrt_ip(r);

@@ -1702,7 +1702,10 @@ DV double low_face_value(const RunView& v, const LowFace& F, int k) {
 // kernel at order 2 without PenteBorne, by SweepFace otherwise), 1 = they
 // are formed here (PenteBorne at orders 1-2), 2 = the run's options decide
 // (batched launches).
-template <int FACES>
+// NB, NC: materials and components known at compile time (plain launches of
+// the usual component counts: unrolled loops, the components in registers),
+// 0 where the run's options decide.
+template <int FACES, int NB = 0, int NC = 0>
 struct SweepUpdateT {
   int sweep;
   // Fused sweeps (PenteBorne, orders 1-2): the faces' flags and integrals
@@ -1719,7 +1722,7 @@ struct SweepUpdateT {
     const bool dirx = (sweep == 1) ? C.x_then_y : !C.x_then_y;
     const long long P = v.pitch, FP = v.fpitch;
     const long long c = (long long)i * v.nx + j;
-    const int ncomp = v.ncomp, nb = v.nbmat;
+    const int ncomp = NC ? NC : v.ncomp, nb = NB ? NB : v.nbmat;
     // Orders 1-2: a cell whose components all come through the first sweep
     // bit for bit unchanged is flagged in u1s instead of having them copied
     // into U1; the second sweep then takes its input from UL (which holds
@@ -1875,7 +1878,9 @@ struct SweepUpdateT {
     // components four at a time: the loads of a group are issued together,
     // ahead of the group's stores (which would otherwise order each
     // component's loads behind the previous component's stores)
-    for (int k0 = 0; k0 < (zface ? 0 : ncomp); k0 += 4) {
+  #pragma unroll (NC ? 4 : 1)
+    for (int k0 = 0; k0 < (NC ? NC : ncomp); k0 += 4) {
+      if (zface) break;
       double qa[4], qb[4], ui[4];
   #pragma unroll
       for (int t = 0; t < 4; ++t) {
@@ -2667,6 +2672,15 @@ __global__ void __launch_bounds__(kBX* kBY) k_sweep_face(RunView v, int sweep) {
 __global__ void __launch_bounds__(kBX* kBY, 7) k_sweep_face3(RunView v, int sweep) { plain_items(v, SweepFaceT<1>{sweep}); }
 __global__ void __launch_bounds__(kBX* kBY) k_sweep_update(RunView v, int sweep) { plain_items(v, SweepUpdateT<0>{sweep}); }
 __global__ void __launch_bounds__(kBX* kBY, 9) k_sweep_update_f(RunView v, int sweep) { plain_items(v, SweepUpdateT<1>{sweep}); }
+// The usual component counts, known at compile time: 1001 x 999 cells moving 124
+// -> 113 us with PenteBorne (2 materials), 1792 x 768 cells at order 3 124 -> 102
+// us (3 materials, Eucclhyd).  Ten resident blocks with PenteBorne (at rest 80 us
+// at 2048 x 2048 cells against 84 with nine), eight without (102 us against 109
+// with six, 107 with nine).
+template <int FACES, int NB, int NC>
+__global__ void __launch_bounds__(kBX* kBY, FACES ? 10 : 8) k_sweep_update_n(RunView v, int sweep) {
+  plain_items(v, SweepUpdateT<FACES, NB, NC>{sweep});
+}
 
 // ------------------------------------------------------- fused remap sweep
 // One launch per sweep for VNR runs with PenteBorne pure at order 2 (the
@@ -2839,6 +2853,26 @@ const char* const kKernelNames[kNumKernelKinds] = {
 // Enqueues one full cycle on stream s; hook(kind) is called before each
 // launch (and with kind = -1 after the last) when given.  Returns the number
 // of kernels.
+// The update kernel of a run: compiled for its materials and components (VNR
+// 3 nbmat + 1, Eucclhyd 3 nbmat + 2), or the general one (conservative
+// projection).
+template <int FACES>
+static void launch_update(const RunView& v, int sweep, dim3 cg, cudaStream_t s) {
+  const dim3 blk(kBX, kBY);
+  const int extra = v.ncomp - 3 * v.nbmat;
+#define UPDATE(NB)                                                                         \
+  if (v.nbmat == NB && extra == 1)                                                         \
+    return k_sweep_update_n<FACES, NB, 3 * NB + 1><<<cg, blk, 0, s>>>(v, sweep);           \
+  if (v.nbmat == NB && extra == 2)                                                         \
+    return k_sweep_update_n<FACES, NB, 3 * NB + 2><<<cg, blk, 0, s>>>(v, sweep);
+  UPDATE(1)
+  UPDATE(2)
+  UPDATE(3)
+#undef UPDATE
+  if (FACES) k_sweep_update_f<<<cg, blk, 0, s>>>(v, sweep);
+  else k_sweep_update<<<cg, blk, 0, s>>>(v, sweep);
+}
+
 // One directional remap sweep (Remap::computeGradPhiFace, computeGradPhi,
 // computeUpwindFaceQuantitiesForProjection, computeUremap) on stream s,
 // shared by both Lagrange schemes.  Returns the number of kernels.
@@ -2883,11 +2917,15 @@ int launch_sweep(const RunView& v, int sweep, cudaStream_t s, const LaunchHook* 
     H(17); k_o3_ystar<<<fg, blk, 0, s>>>(v, sweep); ++nk;
     H(5); k_sweep_face3<<<fg, blk, 0, s>>>(v, sweep); ++nk;
     if (before) before(1);
-    H(6); k_sweep_update<<<cg, blk, 0, s>>>(v, sweep); ++nk;
+    H(6);
+    launch_update<0>(v, sweep, cg, s);
+    ++nk;
   } else if (v.pb == 1) {
     // PenteBorne, orders 1-2: the update forms its face values
     if (before) before(1);
-    H(6); k_sweep_update_f<<<cg, blk, 0, s>>>(v, sweep); ++nk;
+    H(6);
+    launch_update<1>(v, sweep, cg, s);
+    ++nk;
   } else {
     // without PenteBorne the slope kernel wrote the order-2 face values; at
     // order 1 (no slopes) the face kernel forms them
@@ -2895,7 +2933,9 @@ int launch_sweep(const RunView& v, int sweep, cudaStream_t s, const LaunchHook* 
       H(5); k_sweep_face<<<fg, blk, 0, s>>>(v, sweep); ++nk;
     }
     if (before) before(1);
-    H(6); k_sweep_update<<<cg, blk, 0, s>>>(v, sweep); ++nk;
+    H(6);
+    launch_update<0>(v, sweep, cg, s);
+    ++nk;
   }
   return nk;
 }
