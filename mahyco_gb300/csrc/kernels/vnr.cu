@@ -188,22 +188,46 @@ DV double cell_dt(const RunView& v, long long c, int i, int j) {
 // Vnr::computeNodeMass (PhaseLagrange.cc:31-48), updateVelocity (:167-197),
 // updateVelocityBoundaryConditions (ConditionsLimites.cc:12-185),
 // updatePosition (:203-208).
+//
+// INNER: the node has four cells, in fixed corners, and takes no boundary
+// condition (no indexed arrays, which would live in local memory); in plain
+// launches the boundary's nodes are in warps of their own (split_node_items).
+// 2048 x 2048 cells at rest 116 -> 78 us, 801 x 41 cells without the remap
+// 27 -> 17 us, 200 x 10 cells 14 -> 12 us.
 struct LagNodes {
-  __device__ __forceinline__ void operator()(const RunView& v, int i, int j) const {
+  template <bool INNER>
+  DV void node(const RunView& v, int i, int j) const {
     const Ctrl& C = *v.ctrl;
-    if (i > v.ny || j > v.nx) return;
     const long long p = (long long)i * (v.nx + 1) + j;
     // cells of node, getCellsOfNode order (CartesianMesh2D.cc:97-108); loc is
     // the node's position in each cell's node list
     long long cells[4];
     int loc[4], k = 0;
-    if (i < v.ny && j < v.nx) { cells[k] = (long long)i * v.nx + j; loc[k++] = 0; }
-    if (i < v.ny && j > 0) { cells[k] = (long long)i * v.nx + j - 1; loc[k++] = 1; }
-    if (i > 0 && j < v.nx) { cells[k] = (long long)(i - 1) * v.nx + j; loc[k++] = 3; }
-    if (i > 0 && j > 0) { cells[k] = (long long)(i - 1) * v.nx + j - 1; loc[k++] = 2; }
+    const long long c00 = (long long)i * v.nx + j;
+    if (INNER) {
+      k = 4;
+      cells[0] = c00; loc[0] = 0;
+      cells[1] = c00 - 1; loc[1] = 1;
+      cells[2] = c00 - v.nx; loc[2] = 3;
+      cells[3] = c00 - v.nx - 1; loc[3] = 2;
+    } else {
+      if (i < v.ny && j < v.nx) { cells[k] = c00; loc[k++] = 0; }
+      if (i < v.ny && j > 0) { cells[k] = c00 - 1; loc[k++] = 1; }
+      if (i > 0 && j < v.nx) { cells[k] = c00 - v.nx; loc[k++] = 3; }
+      if (i > 0 && j > 0) { cells[k] = c00 - v.nx - 1; loc[k++] = 2; }
+    }
+#define NODE_CELLS(t) _Pragma("unroll") for (int t = 0; t < 4; ++t) if (INNER || t < k)
+    double mc[4], pc[4], qc[4];
+    NODE_CELLS(t) {
+      mc[t] = v.cell_mass[cells[t]];
+      pc[t] = v.p[cells[t]];
+      qc[t] = v.q[cells[t]];
+    }
     // sums from 0.0: first addition as plus_zero (k >= 1 cells)
-    double msum = plus_zero(v.cell_mass[cells[0]]);
-    for (int t = 1; t < k; ++t) msum = msum + v.cell_mass[cells[t]];
+    double msum = plus_zero(mc[0]);
+    NODE_CELLS(t) {
+      if (t > 0) msum = msum + mc[t];
+    }
     const double m = div_pow2(msum, k);  // msum / k, k in {1, 2, 4}
 
     double ux = v.u[p], uy = v.u[v.npitch + p];
@@ -233,17 +257,39 @@ struct LagNodes {
       // the Euler one at every cycle's start and the set-up stored them;
       // without it (Vnr::computeCornerNormal, PhaseLagrange.cc:114-136, at
       // each cycle's start) they come from the current positions of the
-      // node and of its successor / predecessor in the cell's node order.
+      // node and of its successor / predecessor in the cell's node order:
+      // (right, up), (up, left), (left, down), (down, right) for the cell's
+      // bottom-left, bottom-right, top-right and top-left node.  A side's
+      // l n towards its predecessor is the negative of the one towards its
+      // successor (a zero's sign is not seen: every sum starts from +0), so
+      // an inner node forms its four sides once (4 roots and 8 quotients
+      // instead of 8 and 16).
       const long long NP = v.npitch, W = v.nx + 1;
+      double e0[4], e1[4];  // sides right, up, left, down
+      if (INNER && v.XN) {
+        const long long nb[4] = {p + 1, p + W, p - 1, p - W};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const double a0 = 0.5 * (v.XN[NP + nb[q]] - X1), a1 = 0.5 * (X0 - v.XN[nb[q]]);
+          const double la = face_len(a0, a1);
+          e0[q] = qdiv(a0, la) * la;
+          e1[q] = qdiv(a1, la) * la;
+        }
+      }
       auto corner = [&](int t, double& C0, double& C1) {
         if (!v.XN) {
           C0 = ld(v.cqs, (2 * loc[t]) * v.pitch + cells[t]);
           C1 = ld(v.cqs, (2 * loc[t] + 1) * v.pitch + cells[t]);
           return;
         }
-        // successor, predecessor: (right, up), (up, left), (left, down),
-        // (down, right) for the cell's bottom-left, bottom-right, top-right
-        // and top-left node
+        if (INNER) {
+          // successor minus predecessor side: loc 0 (right, up), 1 (up,
+          // left), 3 (down, right), 2 (left, down)
+          constexpr int nx_[4] = {0, 1, 3, 2}, pv_[4] = {1, 2, 0, 3};
+          C0 = e0[nx_[t]] - e0[pv_[t]];
+          C1 = e1[nx_[t]] - e1[pv_[t]];
+          return;
+        }
         const long long nxt[4] = {p + 1, p + W, p - 1, p - W};
         const long long prv[4] = {p + W, p - 1, p - W, p + 1};
         const long long a = nxt[loc[t]], b = prv[loc[t]];
@@ -258,11 +304,10 @@ struct LagNodes {
       auto force = [&](bool sym, double sx, double sy, double& r0, double& r1) {
         r0 = 0.0;
         r1 = 0.0;
-        for (int t = 0; t < k; ++t) {
-          const long long c = cells[t];
+        NODE_CELLS(t) {
           double C0, C1;
           corner(t, C0, C1);
-          const double w = addz(v.p[c], v.q[c]);
+          const double w = addz(pc[t], qc[t]);
           double t0, t1;
           if (!sym) {
             t0 = w * C0;
@@ -280,107 +325,72 @@ struct LagNodes {
         }
       };
       const double u0x = ux, u0y = uy;
-      const bool inner = i > 0 && i < v.ny && j > 0 && j < v.nx;
-      // one pressure in the four cells around an inner node whose corner
-      // normals cancel exactly (nsym, set up with the derivation): the force
-      // sum is +0 without the products.  The four p + q are compared where
-      // the sums are exact on the integer pipe (p or q a zero); elsewhere the
-      // products run, and give the same +0.
-      bool zero = false;
-      if (inner && !v.XN && ld_u8(v.nsym, p)) {  // a flag of the Euler mesh
-        constexpr unsigned long long kMod = 1523ull << 52;  // 2^500
-        unsigned long long w0 = 0ull, w = 0ull;
-        zero = addz_bits(v.p[cells[0]], v.q[cells[0]], w0) && (w0 & kMag) < kMod;
-  #pragma unroll
-        for (int t = 1; t < 4; ++t)
-          zero = zero && addz_bits(v.p[cells[t]], v.q[cells[t]], w) && w == w0;
-      }
-      // An inner node at rest: a zero force sum, so s = dt / m is not formed
-      // (s * (+0) = +0); a zero velocity, (+-0) + (+0) = +0; dt^{n+1}
-      // positive and finite, so X + dt^{n+1} * (+0) = X + (+0) is X (+0 for a
-      // zero X, X not NaN).  One branch for the whole node: the general
-      // path's FP64 operations, if-converted, would be issued for it too.
-      const bool rest = zero && s_easy && ((ubits(u0x) | ubits(u0y)) & kMag) == 0 &&
-                        pos(C.dt_np1) && is_finite(C.dt_np1) && !is_nan(X0) && !is_nan(X1);
-      if (rest) {
-        ux = 0.0;
-        uy = 0.0;
-        xl0 = iszero(X0) ? 0.0 : X0;
-        xl1 = iszero(X1) ? 0.0 : X1;
+      if (INNER) {
+        // one pressure in the four cells around an inner node whose corner
+        // normals cancel exactly (nsym, set up with the derivation): the force
+        // sum is +0 without the products.  The four p + q are compared where
+        // the sums are exact on the integer pipe (p or q a zero); elsewhere the
+        // products run, and give the same +0.
+        bool zero = false;
+        if (!v.XN && ld_u8(v.nsym, p)) {  // a flag of the Euler mesh
+          constexpr unsigned long long kMod = 1523ull << 52;  // 2^500
+          unsigned long long w0 = 0ull, w = 0ull;
+          zero = addz_bits(pc[0], qc[0], w0) && (w0 & kMag) < kMod;
+#pragma unroll
+          for (int t = 1; t < 4; ++t) zero = zero && addz_bits(pc[t], qc[t], w) && w == w0;
+        }
+        // An inner node at rest: a zero force sum, so s = dt / m is not formed
+        // (s * (+0) = +0); a zero velocity, (+-0) + (+0) = +0; dt^{n+1}
+        // positive and finite, so X + dt^{n+1} * (+0) = X + (+0) is X (+0 for a
+        // zero X, X not NaN).  One branch for the whole node: the general
+        // path's FP64 operations, if-converted, would be issued for it too.
+        const bool rest = zero && s_easy && ((ubits(u0x) | ubits(u0y)) & kMag) == 0 &&
+                          pos(C.dt_np1) && is_finite(C.dt_np1) && !is_nan(X0) && !is_nan(X1);
+        if (rest) {
+          ux = 0.0;
+          uy = 0.0;
+          xl0 = iszero(X0) ? 0.0 : X0;
+          xl1 = iszero(X1) ? 0.0 : X1;
+        } else {
+          double r0 = 0.0, r1 = 0.0;
+          if (!zero) force(false, 0., 0., r0, r1);
+          ux = addz(u0x, step(r0));
+          uy = addz(u0y, step(r1));
+          xl0 = addz(X0, mulz(C.dt_np1, ux));
+          xl1 = addz(X1, mulz(C.dt_np1, uy));
+        }
         if (v.vout) {  // m_x/y_velocity, inner nodes only (PhaseLagrange.cc:193)
           v.vout[p] = ux;
           v.vout[v.npitch + p] = uy;
         }
       } else {
-        double r0, r1;
-        if (inner) {
-          if (zero) {
-            r0 = 0.0;
-            r1 = 0.0;
-          } else {
-            force(false, 0., 0., r0, r1);
-          }
-          ux = addz(u0x, step(r0));
-          uy = addz(u0y, step(r1));
-          if (v.vout) {
-            v.vout[p] = ux;
-            v.vout[v.npitch + p] = uy;
-          }
-        }
-        // sides in the reference's order: bottom, top, left, right
-        if (i == 0) {
-          if (v.bc_bottom == kBcSym) {
-            force(true, 1.0, 0.0, r0, r1);
-            ux = addz(u0x, step(r0));
-            uy = addz(u0y, step(r1));
-          } else if (v.bc_bottom == kBcImposed) {
-            ux = v.v_bottom[0];
-            uy = v.v_bottom[1];
-          }
-        }
-        if (i == v.ny) {
-          if (v.bc_top == kBcSym) {
-            force(true, 1.0, 0.0, r0, r1);
-            ux = addz(u0x, step(r0));
-            uy = addz(u0y, step(r1));
-          } else if (v.bc_top == kBcImposed) {
-            ux = v.v_top[0];
-            uy = v.v_top[1];
-          }
-        }
-        if (j == 0) {
-          if (v.bc_left == kBcSym) {
-            force(true, 0.0, 1.0, r0, r1);
-            ux = addz(u0x, step(r0));
-            uy = addz(u0y, step(r1));
-          } else if (v.bc_left == kBcImposed) {
-            ux = v.v_left[0];
-            uy = v.v_left[1];
-          }
-        }
-        if (j == v.nx) {
-          if (v.bc_right == kBcSym) {
-            force(true, 0.0, 1.0, r0, r1);
-            ux = addz(u0x, step(r0));
-            uy = addz(u0y, step(r1));
-          } else if (v.bc_right == kBcImposed) {
-            ux = v.v_right[0];
-            uy = v.v_right[1];
-          }
-        }
-        // corners (ConditionsLimites.cc:133-184)
         const bool top = (i == v.ny), bot = (i == 0), lft = (j == 0), rgt = (j == v.nx);
-        if ((top || bot) && (lft || rgt)) {
-          const int bv = top ? v.bc_top : v.bc_bottom;
-          const int bh = lft ? v.bc_left : v.bc_right;
-          const double vh0 = lft ? v.v_left[0] : v.v_right[0];
-          const double vh1 = lft ? v.v_left[1] : v.v_right[1];
-          if (bv == kBcSym && bh == kBcSym) {
-            ux = 0.0;
-            uy = 0.0;
-          } else if (bv == kBcImposed && bh == kBcImposed) {
-            ux = vh0;
-            uy = vh1;
+        const int bv = top ? v.bc_top : v.bc_bottom, bh = lft ? v.bc_left : v.bc_right;
+        const bool corner_node = (top || bot) && (lft || rgt);
+        // corners (ConditionsLimites.cc:133-184): two symmetry sides or two
+        // imposed ones decide the velocity whatever the sides' own rules give
+        if (corner_node && bv == kBcSym && bh == kBcSym) {
+          ux = 0.0;
+          uy = 0.0;
+        } else if (corner_node && bv == kBcImposed && bh == kBcImposed) {
+          ux = lft ? v.v_left[0] : v.v_right[0];
+          uy = lft ? v.v_left[1] : v.v_right[1];
+        } else {
+          // sides in the reference's order, bottom, top, left, right: a later
+          // one's velocity replaces an earlier one's; a symmetry side's from
+          // the node's old velocity and its force, along the bottom / top
+          // sides' axis (1, 0), the left / right ones' (0, 1)
+          const int bc_v = (top || bot) ? bv : 0, bc_h = (lft || rgt) ? bh : 0;
+          const bool along_h = bc_h == kBcSym || bc_h == kBcImposed;
+          const int bc = along_h ? bc_h : bc_v;
+          if (bc == kBcSym) {
+            double r0, r1;
+            force(true, along_h ? 0.0 : 1.0, along_h ? 1.0 : 0.0, r0, r1);
+            ux = addz(u0x, step(r0));
+            uy = addz(u0y, step(r1));
+          } else if (bc == kBcImposed) {
+            ux = along_h ? (lft ? v.v_left[0] : v.v_right[0]) : (top ? v.v_top[0] : v.v_bottom[0]);
+            uy = along_h ? (lft ? v.v_left[1] : v.v_right[1]) : (top ? v.v_top[1] : v.v_bottom[1]);
           }
         }
         xl0 = addz(X0, mulz(C.dt_np1, ux));
@@ -392,9 +402,19 @@ struct LagNodes {
       xl0 = addz(X0, mulz(C.dt_np1, ux));
       xl1 = addz(X1, mulz(C.dt_np1, uy));
     }
+#undef NODE_CELLS
     v.node_mass[p] = m;
     v.XL[p] = xl0;
     v.XL[v.npitch + p] = xl1;
+  }
+  // out of line: the inner nodes' registers are not spent on it
+  static __device__ __noinline__ void edge_node(const RunView& v, int i, int j) {
+    LagNodes{}.node<false>(v, i, j);
+  }
+  __device__ __forceinline__ void operator()(const RunView& v, int i, int j) const {
+    if (i > v.ny || j > v.nx) return;
+    if (i > 0 && i < v.ny && j > 0 && j < v.nx) node<true>(v, i, j);
+    else edge_node(v, i, j);
   }
 };
 
@@ -1716,6 +1736,22 @@ struct SweepUpdateT {
   const double *tr = nullptr, *tv = nullptr;
   int lc = 0, lm = 0, lp = 0, ts = 0;
   bool phi2 = false;
+  // the mixed / pure flags from the cell's Phi after the first sweep
+  static DV void set_pure(const RunView& v, int nb, long long c, const double* Pr) {
+    int matcell = 0, imatpure = -1;
+    for (int m = 0; m < nb; m++)
+      if (pos(Pr[m * v.pitch + c])) {
+        matcell++;
+        imatpure = m;
+      }
+    if (matcell > 1) {
+      v.mixte[c] = 1;
+      v.pure[c] = -1;
+    } else {
+      v.mixte[c] = 0;
+      v.pure[c] = imatpure;
+    }
+  }
   __device__ __forceinline__ void operator()(const RunView& v, int i, int j) const {
     const Ctrl& C = *v.ctrl;
     if (i >= v.ny || j >= v.nx) return;
@@ -1732,6 +1768,32 @@ struct SweepUpdateT {
     const bool lowo = v.order <= 2;
     const bool from_ul = (sweep == 2) && lowo && v.u1s[c] != 0;
     const double* Uin = (sweep == 1 || from_ul) ? v.UL : v.U1;
+    // A VNR cell at rest (both faces' integrals flagged +0.0 on both sides,
+    // no boundary flux, the Cartesian normals -1 / +1, lengths and rL finite
+    // and not negative): the zero-face path below, which stores no component,
+    // with every sign known (a face's flux is the zero of its coefficient,
+    // whose sign is its normal's; times the normal +0), decided from three
+    // flag bytes ahead of everything else: 81 -> 45 us at 2048 x 2048 cells.
+    if (FACES == 1 && !tz && lowo && v.scheme == HYDRO_SCHEME_VNR && !v.flux_bc &&
+        !C.nout_general && (sweep == 1 || from_ul)) {
+      const long long st = dirx ? 1 : v.nx;
+      const int q = dirx ? j : i, n = dirx ? v.nx : v.ny;
+      unsigned z = v.pbz[c];
+      if (q > 0) z &= v.pbz[c - st];
+      if (q < n - 1) z &= v.pbz[c + st];
+      const double l = dirx ? ld(v.flv, i) : ld(v.flh, j);
+      const bool share = v.dual_method != 2;
+      const double r = (share && v.dual_method == 1) ? v.rL[c] : 0.;
+      if ((z & 3) == 3 && q > 0 && q < n - 1 && (ubits(l) < kInfBits) && (ubits(r) < kInfBits)) {
+        if (share)
+          for (int m = 0; m < nb; ++m) v.FFd[m * P + c] = 0.0;
+        if (sweep == 1) {
+          v.u1s[c] = 1;
+          set_pure(v, nb, c, v.Phi);
+        }
+        return;
+      }
+    }
     const double dt = C.dt_n;
     // PenteBorne, known at compile time for the kernel that forms its faces
     const int pbv = (FACES == 1) ? 1 : v.pb;
@@ -2013,19 +2075,7 @@ struct SweepUpdateT {
         for (int k = 0; k < ncomp; ++k) Phi[k * P + c] = qdiv_shared(Sv, U[k]);
       }
       const double* Pr = keep ? v.Phi : Phi;  // the cell's Phi after the sweep
-      int matcell = 0, imatpure = -1;
-      for (int m = 0; m < nb; m++)
-        if (pos(Pr[m * P + c])) {
-          matcell++;
-          imatpure = m;
-        }
-      if (matcell > 1) {
-        v.mixte[c] = 1;
-        v.pure[c] = -1;
-      } else {
-        v.mixte[c] = 0;
-        v.pure[c] = imatpure;
-      }
+      set_pure(v, nb, c, Pr);
     }
   }
 };
@@ -2613,13 +2663,27 @@ struct LagCellsLagrangeOnly {
       const long long c = (long long)i * v.nx + j, NP = v.npitch;
       const long long n0 = (long long)i * (v.nx + 1) + j;
       const long long nd[4] = {n0, n0 + 1, n0 + v.nx + 2, n0 + v.nx + 1};
-      double uc = 0.0;
+      // the reference multiplies the mean nodal speed by A = 0: +0 for
+      // moderate velocities, so the four roots are not formed
+      unsigned long long big = 0;
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const double a = v.u[nd[k]], b = v.u[NP + nd[k]];
-        uc += sqrt_ip(a * a + b * b) * 0.25;
+        const unsigned long long a = ubits(v.u[nd[k]]) & kMag, b = ubits(v.u[NP + nd[k]]) & kMag;
+        big = a > big ? a : big;
+        big = b > big ? b : big;
       }
-      const double d = div_ip(0.1 * sqrt_ip(v.vL[c]), 0. * uc + v.c[c]);
+      double den;
+      if (big < (1523ull << 52)) {  // 2^500
+        den = plus_zero(v.c[c]);
+      } else {
+        double uc = 0.0;
+        for (int k = 0; k < 4; ++k) {
+          const double a = v.u[nd[k]], b = v.u[NP + nd[k]];
+          uc += sqrt_ip(a * a + b * b) * 0.25;
+        }
+        den = 0. * uc + v.c[c];
+      }
+      const double d = div_ip(0.1 * sqrt_ip(v.vL[c]), den);
       if (v.sans_lagrange == 0 && !is_nan(d)) dtb = ord_bits(d);
       const double p = v.p[c];
       if (!is_nan(p)) pb = ord_bits(p);
@@ -2649,7 +2713,7 @@ __device__ __forceinline__ void plain_items(const RunView& v, const F& f) {
   f(v, blockIdx.y * kBY + threadIdx.y, blockIdx.x * kBX + threadIdx.x);
 }
 
-__global__ void __launch_bounds__(kBX* kBY, 10) k_lag_nodes(RunView v) { plain_items(v, LagNodes{}); }
+__global__ void __launch_bounds__(kBX* kBY, 10) k_lag_nodes(RunView v) { split_node_items(v, LagNodes{}); }
 __global__ void __launch_bounds__(kBX* kBY, 8) k_lag_cells(RunView v) { plain_items(v, LagCells{}); }
 __global__ void __launch_bounds__(kBX* kBY) k_lag_cells_lo(RunView v) { plain_items(v, LagCellsLagrangeOnly{}); }
 __global__ void __launch_bounds__(kBX* kBY) k_next_positions(RunView v) { plain_items(v, NextPositions{}); }
@@ -2969,7 +3033,7 @@ int launch_cycle(const RunView& v, cudaStream_t s, const LaunchHook* hook,
     if (hook) (*hook)(kind);
   };
   H(0); k_begin<<<1, 1, 0, s>>>(v); ++nk;
-  H(2); k_lag_nodes<<<ng, blk, 0, s>>>(v); ++nk;
+  H(2); k_lag_nodes<<<split_node_grid(v), blk, 0, s>>>(v); ++nk;
   if (v.projection == 0) {
     // the Lagrange phase only: its cell kernel reduces the next dt, and the
     // new positions are carried to the next cycle after the loop test
