@@ -2168,62 +2168,40 @@ struct DualUpdate {
     const int ax = dirx ? 0 : 1;
     // inner faces of the sweep through this node (Vertical/HorizontalFaceOfNode,
     // remap/UtilesMesh.cc:53-108): for an x sweep the vertical faces below and
-    // above the node, for a y sweep the horizontal faces left and right of it.
-    // cplus[s] / cminus[s]: the cells right/above and left/below of face s.
-    long long cplus[2], cminus[2];
-    int nface = 0;
-    if (dirx) {
-      if (j >= 1 && j <= v.nx - 1) {
-        if (i >= 1) {
-          cminus[nface] = (long long)(i - 1) * v.nx + j - 1;
-          cplus[nface++] = (long long)(i - 1) * v.nx + j;
-        }
-        if (i <= v.ny - 1) {
-          cminus[nface] = (long long)i * v.nx + j - 1;
-          cplus[nface++] = (long long)i * v.nx + j;
-        }
-      }
-    } else {
-      if (i >= 1 && i <= v.ny - 1) {
-        if (j >= 1) {
-          cminus[nface] = (long long)(i - 1) * v.nx + j - 1;
-          cplus[nface++] = (long long)i * v.nx + j - 1;
-        }
-        if (j <= v.nx - 1) {
-          cminus[nface] = (long long)(i - 1) * v.nx + j;
-          cplus[nface++] = (long long)i * v.nx + j;
-        }
-      }
-    }
-    // mass fluxes through the node's dual faces; when every share is a
-    // zero, each sum below is +0 (sums from 0.0 of zeros)
+    // above the node, for a y sweep the horizontal faces left and right of it
+    // (the second one's cells a row / a column on).  The cells right / above
+    // and left / below of face 0 are pc0, mc0.
+    const long long c00 = (long long)i * v.nx + j;
+    const bool has0 = dirx ? (j >= 1 && j <= v.nx - 1 && i >= 1)
+                           : (i >= 1 && i <= v.ny - 1 && j >= 1);
+    const bool has1 = dirx ? (j >= 1 && j <= v.nx - 1 && i <= v.ny - 1)
+                           : (i >= 1 && i <= v.ny - 1 && j <= v.nx - 1);
+    const long long pc0 = dirx ? c00 - v.nx : c00 - 1, mc0 = c00 - v.nx - 1;
+    const long long pc1 = c00, mc1 = dirx ? c00 - 1 : c00 - v.nx;
+    const int nface = (has0 ? 1 : 0) + (has1 ? 1 : 0);
+    // mass fluxes through the node's dual faces: per material the sum from 0.0
+    // over the faces (0.0 + w0 + w1; a missing face's w a zero), divided by
+    // twice their number (the number with PenteBorne's flux), summed from 0.0
+    // over the materials.  A material whose shares are all zeros adds +0 and
+    // is passed over.  (The faces as a counted list were indexed arrays in local
+    // memory: 87 -> 79 us moving at 1001 x 999 cells, 93 -> 84 us at rest at
+    // 2048 x 2048.)
     const double* W = (v.dual_method == 2) ? v.DPF : v.FFd;  // FFd: each cell's share
-    unsigned long long wor = 0;
-    for (int m = 0; m < nb; ++m)
-      for (int s = 0; s < nface; ++s)
-        wor |= ubits(W[m * P + cplus[s]]) | ubits(W[m * P + cminus[s]]);
-    const bool fzero = (wor & kMag) == 0;
+    const int dv = (v.dual_method == 2) ? nface : 2 * nface;
     double Fp = 0., Fm = 0.;
-    for (int m = 0; m < nb && !fzero; ++m) {
-      // sums from 0.0: the first addition is plus_zero (integer pipe)
-      double pp = 0., pm = 0.;
-      for (int s = 0; s < nface; ++s) {
-        const long long a = cplus[s], b = cminus[s];
-        const double wa = W[m * P + a], wb = W[m * P + b];
-        pp = (s == 0) ? plus_zero(wa) : pp + wa;
-        pm = (s == 0) ? plus_zero(wb) : pm + wb;
-      }
-      if (v.dual_method == 2) {
-        if (nface != 0) {
-          pp = div_pow2(pp, nface);
-          pm = div_pow2(pm, nface);
-        }
-      } else if (nface != 0) {
-        pp = div_pow2(pp, 2 * nface);
-        pm = div_pow2(pm, 2 * nface);
-      }
-      Fp = (m == 0) ? plus_zero(pp) : Fp + pp;
-      Fm = (m == 0) ? plus_zero(pm) : Fm + pm;
+    bool fzero = true;
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      if (m >= nb) break;
+      const double* Wm = W + m * P;
+      const double wp0 = has0 ? Wm[pc0] : 0., wm0 = has0 ? Wm[mc0] : 0.;
+      const double wp1 = has1 ? Wm[pc1] : 0., wm1 = has1 ? Wm[mc1] : 0.;
+      if (((ubits(wp0) | ubits(wm0) | ubits(wp1) | ubits(wm1)) & kMag) == 0) continue;
+      const double pp = div_pow2(plus_zero(wp0) + wp1, dv);
+      const double pm = div_pow2(plus_zero(wm0) + wm1, dv);
+      Fp = fzero ? plus_zero(pp) : Fp + pp;
+      Fm = fzero ? plus_zero(pm) : Fm + pm;
+      fzero = false;
     }
     // previous nodal conserved values and DualPhi
     const double* D = (sweep == 1) ? v.u : v.DPv;
@@ -2855,7 +2833,7 @@ __global__ void __launch_bounds__(kBatchThreads, 8) kb_sweep_grad_nopb(BatchArgs
 __global__ void __launch_bounds__(kBatchThreads) kb_sweep_face(BatchArgs b) { batch_items(b, SweepFaceT<3>{b.sweep}); }
 __global__ void __launch_bounds__(kBatchThreads, 8) kb_sweep_update(BatchArgs b) { batch_items(b, SweepUpdateT<2>{b.sweep}); }
 __global__ void __launch_bounds__(kBatchThreads, 10) kb_dual_grad(BatchArgs b) { batch_items(b, DualGrad{b.sweep}, HYDRO_SCHEME_VNR); }
-__global__ void __launch_bounds__(kBatchThreads, 12) kb_dual_update(BatchArgs b) { batch_items(b, DualUpdate{b.sweep}, HYDRO_SCHEME_VNR); }
+__global__ void __launch_bounds__(kBatchThreads, 10) kb_dual_update(BatchArgs b) { batch_items(b, DualUpdate{b.sweep}, HYDRO_SCHEME_VNR); }
 __global__ void __launch_bounds__(kBatchThreads, 7) kb_final(BatchArgs b) { batch_items(b, Final{}, HYDRO_SCHEME_VNR); }
 
 // One thread per VNR run: cycle start (begin + reduction reset) and cycle
