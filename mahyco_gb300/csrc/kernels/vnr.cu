@@ -440,6 +440,13 @@ static __device__ __noinline__ double void_energy(unsigned mask, double e, doubl
   return e;
 }
 
+// NB, PBV: materials and PenteBorne known at compile time, with the remap and
+// the Lagrange phase (plain launches: the kernel is large enough that its
+// instructions miss the cache, so each run takes code without the other
+// options': at rest 303 -> 268 us at 2048 x 2048 cells, 62 -> 53 us at 403 x 257,
+// eight blocks per SM fastest of seven to ten); 0 / -1 where the run's options
+// decide.
+template <int NB = 0, int PBV = -1>
 struct LagCells {
   __device__ __forceinline__ void operator()(const RunView& v, int i, int j) const {
     Ctrl& C = *v.ctrl;
@@ -466,7 +473,7 @@ struct LagCells {
     // hold the rest geometry, stored when the cell was last found at rest;
     // a cell at rest again then needs only the volume from it, and stores
     // none of them
-    const bool held = v.gL && v.projection == 1 && v.gL[c] != 0;
+    const bool held = v.gL && (NB || v.projection == 1) && v.gL[c] != 0;
     if (rest) {
       g0v[0] = ld(v.geo0, c);
       if (!held) {
@@ -492,7 +499,9 @@ struct LagCells {
       G = vnr_cell_geometry(X, v.order > 1);
     }
     const double vol = G.vol;
-    const int nb = v.nbmat;
+    const int nb = NB ? NB : v.nbmat;
+    const int pbv = PBV < 0 ? v.pb : PBV;
+    const int projection = NB ? 1 : v.projection, sans_lagrange = NB ? 0 : v.sans_lagrange;
     const double thr = v.threshold;
     double f[3], mf[3] = {0., 0., 0.}, rhom_new[3], rho_o[3], em_o[3], pm_o[3], qm_o[3];
     double rho_new = 0.;
@@ -503,7 +512,7 @@ struct LagCells {
     // sum of the sub-volumes at the cycle's start (the pseudo-viscosity's
     // volume): the Euler cell's with the remap, the Lagrangian volume of the
     // previous cycle (vL) without it
-    const double vol_start = (v.projection == 0) ? v.vL[c] : 0.0;
+    const double vol_start = (projection == 0) ? v.vL[c] : 0.0;
     // A cell holding one material p (f = mf = 1 for it, +0 for the others,
     // whose densities are finite and at most the threshold), with the
     // remap, perfect gases only, a threshold in [0, 1), a positive finite
@@ -515,7 +524,7 @@ struct LagCells {
     // the loops' shortcuts are if-converted into FP64 instructions that run
     // for every material.
     int p = -1;
-    bool single = v.projection == 1 && v.sans_lagrange == 0 && nonneg(thr) && dlt(thr, 1.0) &&
+    bool single = projection == 1 && sans_lagrange == 0 && nonneg(thr) && dlt(thr, 1.0) &&
                   pos(vol) && is_finite(vol) && !neg(c_old);
     double fa[3] = {0., 0., 0.}, mfa[3] = {0., 0., 0.}, rma[3] = {0., 0., 0.};
   #pragma unroll
@@ -561,7 +570,7 @@ struct LagCells {
       rho_new = (m == 0) ? plus_zero(fr) : addz(rho_new, fr);
     }
     double e_new, q_new;
-    if (v.sans_lagrange == 0) {
+    if (sans_lagrange == 0) {
       const double rdt = C.rdt_np1;
       // A density that came through the Lagrange phase bit for bit unchanged,
       // positive and within [2^-1000, 2^1001) (so 1/rho is a positive finite
@@ -591,8 +600,8 @@ struct LagCells {
         // flow has not arrived (0 / tau)
         divu_new = qdiv(rdt * (same_rho ? 0.0 : irho_new - irho_old), tau);
         if (neg(divu_old)) {
-          const double s0 = (v.projection == 0) ? vol_start : ld(v.s0, c);
-          const double sq0 = (v.projection == 0) ? sqrt_ip(vol_start) : ld(v.sqs0, c);
+          const double s0 = (projection == 0) ? vol_start : ld(v.s0, c);
+          const double sq0 = (projection == 0) ? sqrt_ip(vol_start) : ld(v.sqs0, c);
           q_new = div_ip(1.0, tau) *
                   (-half(sq0) * c_old * divu_new +
                    v.hgs1 * s0 * divu_new * divu_new);
@@ -707,7 +716,7 @@ struct LagCells {
                                          em_new[1], em_new[2]);
       st_if_new(v.c + c, c_old, cc);
       st_if_new(v.sarg + c, sarg_old, sarg_new);
-      if (v.projection == 0) {
+      if (projection == 0) {
         // Without the remap no later kernel forms the state after this
         // phase: its densities, energies, pseudo-viscosity, and the
         // pressures of computeEOSGP ((gamma - 1) rho e; a Void material
@@ -761,7 +770,7 @@ struct LagCells {
       v.UL[(2 * nb + mat(m)) * P + c] = ue[m];
     }
     v.UL[3 * nb * P + c] = uq;
-    if (v.pb == 1) {
+    if (pbv == 1) {
       double sv = plus_zero(uv[0]);
   #pragma unroll
       for (int m = 1; m < 3; ++m)
@@ -806,8 +815,8 @@ struct LagCells {
           v.UL[(nb + m) * P + c] = zm;
           v.UL[(2 * nb + m) * P + c] = ze;
           v.Phi[m * P + c] = 0.0;
-          v.Phi[(nb + m) * P + c] = (v.pb == 1) ? 0.0 : zm;
-          v.Phi[(2 * nb + m) * P + c] = (v.pb == 1) ? 0.0 : ze;
+          v.Phi[(nb + m) * P + c] = (pbv == 1) ? 0.0 : zm;
+          v.Phi[(2 * nb + m) * P + c] = (pbv == 1) ? 0.0 : ze;
         }
       } else {
         const double zm = mulz(0.0, rho_new), ze = mulz(mulz(0.0, rho_new), e_new);
@@ -820,9 +829,9 @@ struct LagCells {
           v.UL[(nb + m) * P + c] = zm;
           v.UL[(2 * nb + m) * P + c] = ze;
           v.Phi[m * P + c] = 0.0;
-          v.Phi[(nb + m) * P + c] = (v.pb == 1) ? 0.0 : qdiv(zm, vol);
+          v.Phi[(nb + m) * P + c] = (pbv == 1) ? 0.0 : qdiv(zm, vol);
           v.Phi[(2 * nb + m) * P + c] =
-              (v.pb == 1) ? (nz(zm) ? qdiv(ze, zm) : 0.0) : qdiv(ze, vol);
+              (pbv == 1) ? (nz(zm) ? qdiv(ze, zm) : 0.0) : qdiv(ze, vol);
         }
       }
     }
@@ -838,7 +847,7 @@ struct LagCells {
         v.Hy[c] = G.hy;
       }
     }
-    if (v.gL && v.projection == 1 && rest != held) v.gL[c] = rest ? 1 : 0;
+    if (v.gL && projection == 1 && rest != held) v.gL[c] = rest ? 1 : 0;
   }
 };
 
@@ -2331,6 +2340,7 @@ struct DualUpdate {
 // FP64 instructions that run anyway.  Moving cells take it like those at
 // rest: FP64 instructions per cell of a moving flow 29 -> 9, 130 -> 74 us at
 // 1001 x 999 cells.
+template <int NB>
 __device__ __forceinline__ bool final_single(const RunView& v, Ctrl& C, long long c, int nb,
                                              double thr, double vol, const double* vn,
                                              const double* Um, const double* Ue, double Uq,
@@ -2404,12 +2414,13 @@ __device__ __forceinline__ bool final_single(const RunView& v, Ctrl& C, long lon
   if (!is_nan(pres)) pb = ord_bits(pres) > pb ? ord_bits(pres) : pb;
   return true;
 }
+template <int NB>
 __device__ __forceinline__ void final_cell(const RunView& v, Ctrl& C, int i,
                                            int j, unsigned long long& dtb,
                                            unsigned long long& pb) {
   const long long P = v.pitch;
   const long long c = (long long)i * v.nx + j;
-  const int nb = v.nbmat;
+  const int nb = NB ? NB : v.nbmat;
   const double thr = v.threshold;
   const double* U = v.UL + c;  // second sweep output
   const double vol = v.euler_volume;
@@ -2436,7 +2447,7 @@ __device__ __forceinline__ void final_cell(const RunView& v, Ctrl& C, int i,
     spd[3] = ld(v.speed, n0 + v.nx + 1);
     cflsq = ld(v.cflsq, c);
   }
-  if (final_single(v, C, c, nb, thr, vol, vn, Um, Ue, Uq, c_in, sarg_in, spd, cflsq, dtb, pb))
+  if (final_single<NB>(v, C, c, nb, thr, vol, vn, Um, Ue, Uq, c_in, sarg_in, spd, cflsq, dtb, pb))
     return;
   // every sum below starts from 0.0 in the reference: its first addition
   // 0.0 + x is plus_zero(x), on the integer pipe (materials 0 .. nb-1, nb >= 1)
@@ -2574,11 +2585,14 @@ __device__ __forceinline__ void final_cell(const RunView& v, Ctrl& C, int i,
   if (!is_nan(p)) pb = ord_bits(p) > pb ? ord_bits(p) : pb;
 }
 
+// NB: as LagCells (at rest 182 -> 161 us at 2048 x 2048 cells, 33 -> 26 us at
+// 403 x 257)
+template <int NB = 0>
 struct Final {
   __device__ __forceinline__ void operator()(const RunView& v, int i, int j) const {
     Ctrl& C = *v.ctrl;
     unsigned long long dtb = ~0ull, pb = 0ull;
-    if (i < v.ny && j < v.nx) final_cell(v, C, i, j, dtb, pb);
+    if (i < v.ny && j < v.nx) final_cell<NB>(v, C, i, j, dtb, pb);
     block_reduce_minmax(dtb, pb, &C);
   }
 };
@@ -2637,7 +2651,7 @@ struct LagCellsLagrangeOnly {
     Ctrl& C = *v.ctrl;
     unsigned long long dtb = ~0ull, pb = 0ull;
     if (i < v.ny && j < v.nx) {
-      LagCells{}(v, i, j);
+      LagCells<>{}(v, i, j);
       const long long c = (long long)i * v.nx + j, NP = v.npitch;
       const long long n0 = (long long)i * (v.nx + 1) + j;
       const long long nd[4] = {n0, n0 + 1, n0 + v.nx + 2, n0 + v.nx + 1};
@@ -2692,7 +2706,9 @@ __device__ __forceinline__ void plain_items(const RunView& v, const F& f) {
 }
 
 __global__ void __launch_bounds__(kBX* kBY, 10) k_lag_nodes(RunView v) { split_node_items(v, LagNodes{}); }
-__global__ void __launch_bounds__(kBX* kBY, 8) k_lag_cells(RunView v) { plain_items(v, LagCells{}); }
+__global__ void __launch_bounds__(kBX* kBY, 8) k_lag_cells(RunView v) { plain_items(v, LagCells<>{}); }
+template <int NB, int PBV>
+__global__ void __launch_bounds__(kBX* kBY, 8) k_lag_cells_n(RunView v) { plain_items(v, LagCells<NB, PBV>{}); }
 __global__ void __launch_bounds__(kBX* kBY) k_lag_cells_lo(RunView v) { plain_items(v, LagCellsLagrangeOnly{}); }
 __global__ void __launch_bounds__(kBX* kBY) k_next_positions(RunView v) { plain_items(v, NextPositions{}); }
 __global__ void __launch_bounds__(kBX* kBY) k_face_grad(RunView v, int sweep) { plain_items(v, FaceGrad{sweep}); }
@@ -2823,10 +2839,11 @@ __global__ void __launch_bounds__(128, 7) k_sweep_fused_y(RunView v, int sweep) 
 __global__ void __launch_bounds__(kBX* kBY, 10) k_dual_grad(RunView v, int sweep) { plain_items(v, DualGrad{sweep}); }
 // ten resident blocks: where nodes are quiet the kernel waits on memory
 __global__ void __launch_bounds__(kBX* kBY, 12) k_dual_update(RunView v, int sweep) { plain_items(v, DualUpdate{sweep}); }
-__global__ void __launch_bounds__(kBX* kBY, 8) k_final(RunView v) { plain_items(v, Final{}); }
+template <int NB>
+__global__ void __launch_bounds__(kBX* kBY, 8) k_final(RunView v) { plain_items(v, Final<NB>{}); }
 
 __global__ void __launch_bounds__(kBatchThreads, 10) kb_lag_nodes(BatchArgs b) { batch_items(b, LagNodes{}, HYDRO_SCHEME_VNR); }
-__global__ void __launch_bounds__(kBatchThreads, 8) kb_lag_cells(BatchArgs b) { batch_items(b, LagCells{}, HYDRO_SCHEME_VNR); }
+__global__ void __launch_bounds__(kBatchThreads, 8) kb_lag_cells(BatchArgs b) { batch_items(b, LagCells<>{}, HYDRO_SCHEME_VNR); }
 __global__ void __launch_bounds__(kBatchThreads) kb_face_grad(BatchArgs b) { batch_items(b, FaceGrad{b.sweep}); }
 __global__ void __launch_bounds__(kBatchThreads, 8) kb_sweep_grad(BatchArgs b) { batch_items(b, SweepGradAny{b.sweep}); }
 __global__ void __launch_bounds__(kBatchThreads, 8) kb_sweep_grad_nopb(BatchArgs b) { batch_items(b, SweepGradNoPB{b.sweep}); }
@@ -2834,7 +2851,7 @@ __global__ void __launch_bounds__(kBatchThreads) kb_sweep_face(BatchArgs b) { ba
 __global__ void __launch_bounds__(kBatchThreads, 8) kb_sweep_update(BatchArgs b) { batch_items(b, SweepUpdateT<2>{b.sweep}); }
 __global__ void __launch_bounds__(kBatchThreads, 10) kb_dual_grad(BatchArgs b) { batch_items(b, DualGrad{b.sweep}, HYDRO_SCHEME_VNR); }
 __global__ void __launch_bounds__(kBatchThreads, 10) kb_dual_update(BatchArgs b) { batch_items(b, DualUpdate{b.sweep}, HYDRO_SCHEME_VNR); }
-__global__ void __launch_bounds__(kBatchThreads, 7) kb_final(BatchArgs b) { batch_items(b, Final{}, HYDRO_SCHEME_VNR); }
+__global__ void __launch_bounds__(kBatchThreads, 7) kb_final(BatchArgs b) { batch_items(b, Final<>{}, HYDRO_SCHEME_VNR); }
 
 // One thread per VNR run: cycle start (begin + reduction reset) and cycle
 // end (Eucclhyd runs of the batch: kbe_begin / kbe_end).
@@ -2984,6 +3001,24 @@ int launch_sweep(const RunView& v, int sweep, cudaStream_t s, const LaunchHook* 
 
 int launch_cycle_euc(const RunView& v, cudaStream_t s, const LaunchHook* hook);
 
+// The Lagrange cell kernel of a run with the remap: compiled for its materials
+// and PenteBorne, or (advection cases) the general one.
+static void launch_lag_cells(const RunView& v, dim3 cg, cudaStream_t s) {
+  const dim3 blk(kBX, kBY);
+  if (v.sans_lagrange == 0 && (v.pb == 0 || v.pb == 1)) {
+#define LAG_CELLS(NB, PBV) \
+  if (v.nbmat == NB && v.pb == PBV) return k_lag_cells_n<NB, PBV><<<cg, blk, 0, s>>>(v);
+    LAG_CELLS(1, 0)
+    LAG_CELLS(1, 1)
+    LAG_CELLS(2, 0)
+    LAG_CELLS(2, 1)
+    LAG_CELLS(3, 0)
+    LAG_CELLS(3, 1)
+#undef LAG_CELLS
+  }
+  k_lag_cells<<<cg, blk, 0, s>>>(v);
+}
+
 // The dual remap's launches that the cell sweeps do not need run on the
 // fork's second stream, when there is one (a captured cycle):
 //   dual_grad 1 (velocities, Lagrange positions)  beside the Lagrange cells
@@ -3026,7 +3061,7 @@ int launch_cycle(const RunView& v, cudaStream_t s, const LaunchHook* hook,
     fork_wait(d, s, fork->ev[0]);
     k_dual_grad<<<ng, blk, 0, d>>>(v, 1); ++nk;
   }
-  H(3); k_lag_cells<<<cg, blk, 0, s>>>(v); ++nk;
+  H(3); launch_lag_cells(v, cg, s); ++nk;
   nk += launch_sweep(v, 1, s, hook, nullptr);
   if (!fork) {
     H(7); k_dual_grad<<<ng, blk, 0, s>>>(v, 1); ++nk;
@@ -3048,7 +3083,11 @@ int launch_cycle(const RunView& v, cudaStream_t s, const LaunchHook* hook,
     fork_wait(s, d, fork->ev[3]);
   }
   H(8); k_dual_update<<<ng, blk, 0, s>>>(v, 2); ++nk;
-  H(9); k_final<<<cg, blk, 0, s>>>(v); ++nk;
+  H(9);
+  if (v.nbmat == 1) k_final<1><<<cg, blk, 0, s>>>(v);
+  else if (v.nbmat == 2) k_final<2><<<cg, blk, 0, s>>>(v);
+  else k_final<3><<<cg, blk, 0, s>>>(v);
+  ++nk;
   H(10); k_end<<<1, 1, 0, s>>>(v); ++nk;
   H(-1);
   return nk;
