@@ -898,8 +898,21 @@ struct FaceGrad {
       ax = 1;
     }
     const double dx = plus_zero(v.XcL[ax * P + front] - v.XcL[ax * P + back]);
-    for (int k = 0; k < v.ncomp; ++k)
-      v.phiG[k * FP + fidx] = qdiv(v.Phi[k * P + front] - v.Phi[k * P + back], dx);
+    // four components at a time, their loads ahead of the stores (batched 92 ->
+    // 80 us for 1.9 M cells)
+    const int ncomp = v.ncomp;
+#pragma unroll 1
+    for (int k0 = 0; k0 < ncomp; k0 += 4) {
+      double a[4], b[4];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        a[t] = (k0 + t < ncomp) ? v.Phi[(k0 + t) * P + front] : 0.;
+        b[t] = (k0 + t < ncomp) ? v.Phi[(k0 + t) * P + back] : 0.;
+      }
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+        if (k0 + t < ncomp) v.phiG[(k0 + t) * FP + fidx] = qdiv(a[t] - b[t], dx);
+    }
   }
 };
 
@@ -1377,16 +1390,29 @@ struct SweepGradNoPB {
     const double* Pc = v.Phi + c;
     const double* Pp = v.Phi + cp;
     const double* Pm = v.Phi + cm;
-    for (int k = 0; k < ncomp; ++k) {
-      const double y0 = Pc[k * P];
-      const double yp = Pp[k * P], ym = Pm[k * P];
-      double gp = 0., gm = 0.;
-      if (has_gp) gp = v.phiG[k * FP + fp];
-      if (has_gm) gm = v.phiG[k * FP + fm];
-      const double grad = limit_grad1(lim, gp, gm, yp, ym, h0, hp, hm);
-      // y0 + s * slope exactly (a zero slope on the integer pipe)
-      if (up_p) v.phiF[k * FP + fp] = addz(y0, mulz(sp, grad));
-      if (up_m) v.phiF[k * FP + fm] = addz(y0, mulz(sm, grad));
+    // two components at a time, their loads ahead of the stores
+#pragma unroll 1
+    for (int k0 = 0; k0 < ncomp; k0 += 2) {
+      double y0[2], yp[2], ym[2], gp[2], gm[2];
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        const int k = k0 + t;
+        const bool in = k < ncomp;
+        y0[t] = in ? Pc[k * P] : 0.;
+        yp[t] = in ? Pp[k * P] : 0.;
+        ym[t] = in ? Pm[k * P] : 0.;
+        gp[t] = (in && has_gp) ? v.phiG[k * FP + fp] : 0.;
+        gm[t] = (in && has_gm) ? v.phiG[k * FP + fm] : 0.;
+      }
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        const int k = k0 + t;
+        if (k >= ncomp) break;
+        const double grad = limit_grad1(lim, gp[t], gm[t], yp[t], ym[t], h0, hp, hm);
+        // y0 + s * slope exactly (a zero slope on the integer pipe)
+        if (up_p) v.phiF[k * FP + fp] = addz(y0[t], mulz(sp, grad));
+        if (up_m) v.phiF[k * FP + fm] = addz(y0[t], mulz(sm, grad));
+      }
     }
   }
 };
@@ -2718,7 +2744,9 @@ __global__ void __launch_bounds__(kBX* kBY) k_face_grad(RunView v, int sweep) { 
 // compiler's eight, k_sweep_face3 179 -> 145 us at seven against five.
 __global__ void __launch_bounds__(kBX* kBY, 12) k_o3_grad(RunView v, int sweep) { plain_items(v, O3Grad{sweep}); }
 __global__ void __launch_bounds__(kBX* kBY, 12) k_o3_ystar(RunView v, int sweep) { plain_items(v, O3Ystar{sweep}); }
-__global__ void __launch_bounds__(kBX* kBY) k_sweep_grad(RunView v, int sweep) { plain_items(v, SweepGradNoPB{sweep}); }
+// 1001 x 999 cells, 2 materials: 126 us at eight blocks per SM, 136 at six, 145
+// at the compiler's five
+__global__ void __launch_bounds__(kBX* kBY, 8) k_sweep_grad(RunView v, int sweep) { plain_items(v, SweepGradNoPB{sweep}); }
 // eight resident blocks: the kernel waits on memory more than it computes
 // at rest; measured faster than the register-limited four to six
 __global__ void __launch_bounds__(kBX* kBY, 8) k_sweep_grad_pb(RunView v, int sweep, int rows,
