@@ -158,13 +158,14 @@ DV double material_sound(const RunView& v, int m, double rm, double pm, long lon
 // The mean-pressure step replaces the sound speed by the mixture's wherever
 // the density is positive, and nothing else reads a material's sound speed:
 // those are formed (and the stored one read) only in the other cells.
+template <int NB = 0>
 struct EucCellPre {
   __device__ __forceinline__ void operator()(const RunView& v, int i, int j) const {
     unsigned long long dtb = ~0ull;
     if (i < v.ny && j < v.nx) {
       const long long P = v.pitch, NP = v.npitch;
       const long long c = (long long)i * v.nx + j;
-      const int nb = v.nbmat;
+      const int nb = NB ? NB : v.nbmat;
       // the inputs, ahead of the stores (which would order later loads
       // behind them)
       double rm[3], em[3], fm[3], mfm[3];
@@ -297,13 +298,14 @@ DV void bc_velocity(int bc, double V0, double V1, const double* Mp, const double
 // 1792 x 768 cells, 3 materials: 472 -> 322 us (five blocks per SM; four to
 // ten within 10 %); with the boundary's nodes in warps of their own 303 us,
 // and 70 x 30 cells 33 -> 22 us.
+template <int NB = 0>
 struct EucNodes {
   template <bool INNER>
   DV void node(const RunView& v, int i, int j) const {
     const Ctrl& C = *v.ctrl;
     const long long P = v.pitch, NP = v.npitch;
     const long long p = (long long)i * (v.nx + 1) + j;
-    const int nb = v.nbmat;
+    const int nb = NB ? NB : v.nbmat;
     // cells of the node in getCellsOfNode order (CartesianMesh2D.cc:97-108)
     // and the node's position in each
     long long cells[4];
@@ -518,7 +520,7 @@ struct EucNodes {
   }
   // out of line: the inner nodes' registers are not spent on it
   static __device__ __noinline__ void edge_node(const RunView& v, int i, int j) {
-    EucNodes{}.node<false>(v, i, j);
+    EucNodes<NB>{}.template node<false>(v, i, j);
   }
 };
 
@@ -538,6 +540,7 @@ struct EucNodes {
 //    for bit, its forces are the cell's and are formed once;
 //  - corner matrices without off-diagonal entries (cmat_diag, see EucNodes);
 //  - every velocity difference at the corners a zero: no matrix product.
+template <int NB = 0>
 struct EucCells {
   // The sub-cell force l (-pe) + M s (u - u_ex) of one corner.
   struct Corner {
@@ -565,7 +568,7 @@ struct EucCells {
                       int p) {
     const Ctrl& C = *v.ctrl;
     const long long P = v.pitch, NP = v.npitch;
-    const int nb = v.nbmat, nbl = NS == 1 ? 1 : nb;
+    const int nb = NB ? NB : v.nbmat, nbl = NS == 1 ? 1 : nb;
     auto mat = [&](int m) { return NS == 1 ? p : m; };
     const double vol = G.vol;
     const double rho = v.rho[c], snd = v.c[c];
@@ -773,7 +776,7 @@ struct EucCells {
     if (i >= v.ny || j >= v.nx) return;
     const long long P = v.pitch, NP = v.npitch;
     const long long c = (long long)i * v.nx + j;
-    const int nb = v.nbmat;
+    const int nb = NB ? NB : v.nbmat;
     const long long n0 = (long long)i * (v.nx + 1) + j;
     const long long nd[4] = {n0, n0 + 1, n0 + v.nx + 2, n0 + v.nx + 1};
     double X[4][2];
@@ -844,6 +847,7 @@ struct EucCells {
 // density or energy) returns false before any store.  One branch for the
 // cell: 35 -> 8 FP64 instructions, 119 -> 72 us at 1792 x 768 cells and 3
 // materials.
+template <int NB = 0>
 struct EucFinal {
   static DV void store_velocity(const RunView& v, long long c, double un0, double un1) {
     // velocities for the outputs (PhaseRemapFinal.cc:200-213): kept where
@@ -859,7 +863,7 @@ struct EucFinal {
   }
   static DV bool single(const RunView& v, long long c) {
     const long long P = v.pitch;
-    const int nb = v.nbmat;
+    const int nb = NB ? NB : v.nbmat;
     const double* U = v.UL + c;
     const double thr = v.threshold;
     if (!(nonneg(thr) && dlt(thr, 1.0))) return false;
@@ -920,7 +924,7 @@ struct EucFinal {
     const long long P = v.pitch;
     const long long c = (long long)i * v.nx + j;
     if (single(v, c)) return;
-    const int nb = v.nbmat;
+    const int nb = NB ? NB : v.nbmat;
     const double thr = v.threshold;
     const double* U = v.UL + c;  // second sweep output
     const double vol = ldg(v.evol, c);
@@ -1060,18 +1064,22 @@ __device__ __forceinline__ void plain_items(const RunView& v, const F& f) {
   f(v, blockIdx.y * kBY + threadIdx.y, blockIdx.x * kBX + threadIdx.x);
 }
 
-__global__ void __launch_bounds__(kBX* kBY, 8) ke_cell_pre(RunView v) { plain_items(v, EucCellPre{}); }
-__global__ void __launch_bounds__(kBX* kBY, 5) ke_nodes(RunView v) { split_node_items(v, EucNodes{}); }
-__global__ void __launch_bounds__(kBX* kBY, 8) ke_cells(RunView v) { plain_items(v, EucCells{}); }
-__global__ void __launch_bounds__(kBX* kBY, 10) ke_final(RunView v) { plain_items(v, EucFinal{}); }
+template <int NB>
+__global__ void __launch_bounds__(kBX* kBY, 8) ke_cell_pre(RunView v) { plain_items(v, EucCellPre<NB>{}); }
+template <int NB>
+__global__ void __launch_bounds__(kBX* kBY, 5) ke_nodes(RunView v) { split_node_items(v, EucNodes<NB>{}); }
+template <int NB>
+__global__ void __launch_bounds__(kBX* kBY, 8) ke_cells(RunView v) { plain_items(v, EucCells<NB>{}); }
+template <int NB>
+__global__ void __launch_bounds__(kBX* kBY, 10) ke_final(RunView v) { plain_items(v, EucFinal<NB>{}); }
 
 // Batched launches of the Eucclhyd phases (the batch's VNR runs are skipped;
 // the remap sweeps are the shared batched kernels of vnr.cu).
 constexpr int kE = HYDRO_SCHEME_EUCCLHYD;
-__global__ void __launch_bounds__(kBatchThreads, 8) kbe_cell_pre(BatchArgs b) { batch_items(b, EucCellPre{}, kE); }
-__global__ void __launch_bounds__(kBatchThreads, 8) kbe_nodes(BatchArgs b) { batch_items(b, EucNodes{}, kE); }
-__global__ void __launch_bounds__(kBatchThreads, 8) kbe_cells(BatchArgs b) { batch_items(b, EucCells{}, kE); }
-__global__ void __launch_bounds__(kBatchThreads, 10) kbe_final(BatchArgs b) { batch_items(b, EucFinal{}, kE); }
+__global__ void __launch_bounds__(kBatchThreads, 8) kbe_cell_pre(BatchArgs b) { batch_items(b, EucCellPre<>{}, kE); }
+__global__ void __launch_bounds__(kBatchThreads, 8) kbe_nodes(BatchArgs b) { batch_items(b, EucNodes<>{}, kE); }
+__global__ void __launch_bounds__(kBatchThreads, 8) kbe_cells(BatchArgs b) { batch_items(b, EucCells<>{}, kE); }
+__global__ void __launch_bounds__(kBatchThreads, 10) kbe_final(BatchArgs b) { batch_items(b, EucFinal<>{}, kE); }
 // one thread per Eucclhyd run: cycle start and end
 __global__ void kbe_begin(const RunView* views, const int* ninst) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1129,7 +1137,8 @@ int batch_occupancy_euc(int* blocks_per_sm) {
 
 // One Eucclhyd cycle on stream s (kind ids: 0 begin, 12 cell_pre, 13 nodes,
 // 14 cells, sweeps, 15 final, 10 end).  Returns the number of kernels.
-int launch_cycle_euc(const RunView& v, cudaStream_t s, const LaunchHook* hook) {
+template <int NB>
+static int launch_cycle_n(const RunView& v, cudaStream_t s, const LaunchHook* hook) {
   const dim3 blk(kBX, kBY);
   const dim3 cg((v.nx + kBX - 1) / kBX, (v.ny + kBY - 1) / kBY);
   int nk = 0;
@@ -1137,14 +1146,20 @@ int launch_cycle_euc(const RunView& v, cudaStream_t s, const LaunchHook* hook) {
     if (hook) (*hook)(kind);
   };
   H(0); ke_begin<<<1, 1, 0, s>>>(v); ++nk;
-  H(12); ke_cell_pre<<<cg, blk, 0, s>>>(v); ++nk;
-  H(13); ke_nodes<<<split_node_grid(v), blk, 0, s>>>(v); ++nk;
-  H(14); ke_cells<<<cg, blk, 0, s>>>(v); ++nk;
+  H(12); ke_cell_pre<NB><<<cg, blk, 0, s>>>(v); ++nk;
+  H(13); ke_nodes<NB><<<split_node_grid(v), blk, 0, s>>>(v); ++nk;
+  H(14); ke_cells<NB><<<cg, blk, 0, s>>>(v); ++nk;
   for (int sweep = 1; sweep <= 2; ++sweep) nk += launch_sweep(v, sweep, s, hook, nullptr);
-  H(15); ke_final<<<cg, blk, 0, s>>>(v); ++nk;
+  H(15); ke_final<NB><<<cg, blk, 0, s>>>(v); ++nk;
   H(10); ke_end<<<1, 1, 0, s>>>(v); ++nk;
   H(-1);
   return nk;
+}
+
+int launch_cycle_euc(const RunView& v, cudaStream_t s, const LaunchHook* hook) {
+  if (v.nbmat == 1) return launch_cycle_n<1>(v, s, hook);
+  if (v.nbmat == 2) return launch_cycle_n<2>(v, s, hook);
+  return launch_cycle_n<3>(v, s, hook);
 }
 
 }  // namespace hydro
