@@ -940,6 +940,10 @@ struct PPCell {
 };
 __device__ __noinline__ PPFluxes pp_fluxes_call(const PPCell g, double thr, double y0, double yp,
                                                 double ym, bool do_ab, bool dual_k) {
+  // a side with a zero swept length is recorded, not stored (pb_zero_sides):
+  // its integral is not read, so it is not formed (in a smooth flow the
+  // outflow leaves a cell through one side)
+  const bool do_a = do_ab && !iszero(g.ppa), do_b = do_ab && !iszero(g.ppb);
   // Remap::computeGradPhiFace{1,2}: (Phi(front) - Phi(back)) / (XcL(front) -
   // XcL(back)); front / back are the plus / minus neighbours along x, the
   // minus / plus ones along y
@@ -949,9 +953,9 @@ __device__ __noinline__ PPFluxes pp_fluxes_call(const PPCell g, double thr, doub
   const double grad = limit_grad1(g.lim, gp, gm, yp, ym, g.h0, g.hp, g.hm);
   const PPShape sh = pp_shape(g.lim, thr, y0, yp, ym, g.h0, g.hp, g.hm, grad);
   PPFluxes r;
-  r.a = do_ab ? pp_integral(sh, half(-g.h0), half(-g.h0) + g.ppa, g.h0, y0, yp, ym, g.ppa) : 0.;
-  r.b = do_ab ? pp_integral(sh, half(g.h0) - g.ppb, half(g.h0), g.h0, y0, yp, ym, g.ppb) : 0.;
-  r.d = dual_k ? pp_integral(sh, 0., g.ppd, g.h0, y0, yp, ym, g.ppd) : 0.;
+  r.a = do_a ? pp_integral(sh, half(-g.h0), half(-g.h0) + g.ppa, g.h0, y0, yp, ym, g.ppa) : 0.;
+  r.b = do_b ? pp_integral(sh, half(g.h0) - g.ppb, half(g.h0), g.h0, y0, yp, ym, g.ppb) : 0.;
+  r.d = (dual_k && !iszero(g.ppd)) ? pp_integral(sh, 0., g.ppd, g.h0, y0, yp, ym, g.ppd) : 0.;
   return r;
 }
 // nonneg((yp - y0) * (ym - y0)): a neighbour with the cell's own bits, all
