@@ -851,6 +851,17 @@ struct LagCells {
   }
 };
 
+// Batched launches: the tile's run decides (uniform over the block); the usual
+// runs take the code compiled for their materials (435 -> 418 us for 40 runs of
+// 1.9 M cells, the final 172 -> 149).
+struct LagCellsAny {
+  __device__ __forceinline__ void operator()(const RunView& v, int i, int j) const {
+    if (v.pb == 0 && v.sans_lagrange == 0 && v.nbmat == 1) LagCells<1, 0>{}(v, i, j);
+    else if (v.pb == 0 && v.sans_lagrange == 0 && v.nbmat == 2) LagCells<2, 0>{}(v, i, j);
+    else LagCells<>{}(v, i, j);
+  }
+};
+
 // Face normal velocity (PrepareRemap.cc:42-63): mean of the two nodes'
 // Lagrange velocities along the face normal; "+ 0.0" is the dot product's
 // zero start for the other axis.
@@ -2627,6 +2638,15 @@ struct Final {
   }
 };
 
+// Batched launches: as LagCellsAny.
+struct FinalAny {
+  __device__ __forceinline__ void operator()(const RunView& v, int i, int j) const {
+    if (v.nbmat == 1) Final<1>{}(v, i, j);
+    else if (v.nbmat == 2) Final<2>{}(v, i, j);
+    else Final<3>{}(v, i, j);
+  }
+};
+
 // Initial reductions (dt candidate and max pressure of the initial state).
 __global__ void __launch_bounds__(kBX* kBY) k_init_reductions(RunView v) {
   Ctrl& C = *v.ctrl;
@@ -2874,16 +2894,20 @@ __global__ void __launch_bounds__(kBX* kBY, 12) k_dual_update(RunView v, int swe
 template <int NB>
 __global__ void __launch_bounds__(kBX* kBY, 8) k_final(RunView v) { plain_items(v, Final<NB>{}); }
 
+// Resident blocks of the batched kernels by timing 5 to 12 on 40 runs of 1.9 M
+// cells: slopes 180 us at ten (191 at eight), face gradients 75 at twelve (81
+// unbounded), update 170 at seven (175 at eight), final 144 at eight (149 at
+// seven), dual update 146 at ten (155 at twelve).
 __global__ void __launch_bounds__(kBatchThreads, 10) kb_lag_nodes(BatchArgs b) { batch_items(b, LagNodes{}, HYDRO_SCHEME_VNR); }
-__global__ void __launch_bounds__(kBatchThreads, 8) kb_lag_cells(BatchArgs b) { batch_items(b, LagCells<>{}, HYDRO_SCHEME_VNR); }
-__global__ void __launch_bounds__(kBatchThreads) kb_face_grad(BatchArgs b) { batch_items(b, FaceGrad{b.sweep}); }
+__global__ void __launch_bounds__(kBatchThreads, 8) kb_lag_cells(BatchArgs b) { batch_items(b, LagCellsAny{}, HYDRO_SCHEME_VNR); }
+__global__ void __launch_bounds__(kBatchThreads, 12) kb_face_grad(BatchArgs b) { batch_items(b, FaceGrad{b.sweep}); }
 __global__ void __launch_bounds__(kBatchThreads, 8) kb_sweep_grad(BatchArgs b) { batch_items(b, SweepGradAny{b.sweep}); }
-__global__ void __launch_bounds__(kBatchThreads, 8) kb_sweep_grad_nopb(BatchArgs b) { batch_items(b, SweepGradNoPB{b.sweep}); }
+__global__ void __launch_bounds__(kBatchThreads, 10) kb_sweep_grad_nopb(BatchArgs b) { batch_items(b, SweepGradNoPB{b.sweep}); }
 __global__ void __launch_bounds__(kBatchThreads) kb_sweep_face(BatchArgs b) { batch_items(b, SweepFaceT<3>{b.sweep}); }
-__global__ void __launch_bounds__(kBatchThreads, 8) kb_sweep_update(BatchArgs b) { batch_items(b, SweepUpdateT<2>{b.sweep}); }
+__global__ void __launch_bounds__(kBatchThreads, 7) kb_sweep_update(BatchArgs b) { batch_items(b, SweepUpdateT<2>{b.sweep}); }
 __global__ void __launch_bounds__(kBatchThreads, 10) kb_dual_grad(BatchArgs b) { batch_items(b, DualGrad{b.sweep}, HYDRO_SCHEME_VNR); }
 __global__ void __launch_bounds__(kBatchThreads, 10) kb_dual_update(BatchArgs b) { batch_items(b, DualUpdate{b.sweep}, HYDRO_SCHEME_VNR); }
-__global__ void __launch_bounds__(kBatchThreads, 7) kb_final(BatchArgs b) { batch_items(b, Final<>{}, HYDRO_SCHEME_VNR); }
+__global__ void __launch_bounds__(kBatchThreads, 8) kb_final(BatchArgs b) { batch_items(b, FinalAny{}, HYDRO_SCHEME_VNR); }
 
 // One thread per VNR run: cycle start (begin + reduction reset) and cycle
 // end (Eucclhyd runs of the batch: kbe_begin / kbe_end).
