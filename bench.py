@@ -134,10 +134,12 @@ def algorithmic_bytes(kind: str, nb: int, pb: bool, rest: bool = False) -> int:
         table["k_lag_cells"] -= 4 + 4 + 5 - 0.125
     if rest and pb:
         # a cell at rest: the node velocity along the sweep in / its flag
-        # byte out; U, 2 node velocities, 2 outer normals and the flag bytes
-        # in / the mass-flux shares (and a flag byte) out
+        # byte out; two flag bytes in (the cell's own integrals', in the second
+        # sweep the unchanged flag), in the first sweep (half of the launches)
+        # the fractions / the mass-flux shares, in the first sweep a flag
+        # byte and the mixed / pure integers out
         table["k_sweep_grad"] = 1.25
-        table["k_sweep_update"] = (nc + 4.25) + (nb + 0.125)
+        table["k_sweep_update"] = (nb / 2 + 0.25) + (nb + 0.5625)
     return int(table.get(kind, 0) * d)
 
 

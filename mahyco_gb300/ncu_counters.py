@@ -32,8 +32,10 @@ def _value(s: str) -> float:
 
 
 def _name(kernel: str) -> str:
+    """k_<kind>; the instances for a run's materials (k_<kind>_n<...>) count
+    as their kind."""
     m = re.search(r"(k_\w+)", kernel)
-    return m.group(1) if m else kernel
+    return re.sub(r"_n$", "", m.group(1)) if m else kernel
 
 
 def read_capture(path: str) -> dict[str, list[dict]]:
