@@ -446,7 +446,10 @@ static __device__ __noinline__ double void_energy(unsigned mask, double e, doubl
 // options': at rest 303 -> 268 us at 2048 x 2048 cells, 62 -> 53 us at 403 x 257,
 // eight blocks per SM fastest of seven to ten); 0 / -1 where the run's options
 // decide.
-template <int NB = 0, int PBV = -1>
+// PROJ: with NB, the remap (1) or the Lagrange phase alone (0), where nothing
+// reads the remap's inputs (conserved values, Phi, centroid, widths) and they
+// are not formed (801 x 41 cells 26 -> 20 us).
+template <int NB = 0, int PBV = -1, int PROJ = 1>
 struct LagCells {
   __device__ __forceinline__ void operator()(const RunView& v, int i, int j) const {
     Ctrl& C = *v.ctrl;
@@ -473,7 +476,7 @@ struct LagCells {
     // hold the rest geometry, stored when the cell was last found at rest;
     // a cell at rest again then needs only the volume from it, and stores
     // none of them
-    const bool held = v.gL && (NB || v.projection == 1) && v.gL[c] != 0;
+    const bool held = v.gL && (NB ? PROJ == 1 : v.projection == 1) && v.gL[c] != 0;
     if (rest) {
       g0v[0] = ld(v.geo0, c);
       if (!held) {
@@ -501,7 +504,7 @@ struct LagCells {
     const double vol = G.vol;
     const int nb = NB ? NB : v.nbmat;
     const int pbv = PBV < 0 ? v.pb : PBV;
-    const int projection = NB ? 1 : v.projection, sans_lagrange = NB ? 0 : v.sans_lagrange;
+    const int projection = NB ? PROJ : v.projection, sans_lagrange = NB ? 0 : v.sans_lagrange;
     const double thr = v.threshold;
     double f[3], mf[3] = {0., 0., 0.}, rhom_new[3], rho_o[3], em_o[3], pm_o[3], qm_o[3];
     double rho_new = 0.;
@@ -748,6 +751,10 @@ struct LagCells {
       // updatePeriodicBoundaryConditions: first and last column take the
       // initial density of the row's first cell
       if (v.periodic_x && (j == v.nx - 1 || j == 0)) rho_new = ld(v.rho0_left, i);
+    }
+    if (projection == 0) {  // no remap: only the volume is read again
+      v.vL[c] = vol;
+      return;
     }
     // ---- PrepareRemap (cell part): the conserved values per material
     // (volume, mass, energy; indexes known at compile time, so they stay in
@@ -2696,12 +2703,13 @@ __global__ void k_node_speed(RunView v) {
 // :14-50: cfl 0.1, the sub-volumes just formed, the new node velocities and
 // sound speed, A = 0) and pressure maximum, which the remap's final kernel
 // reduces otherwise.
+template <int NB>
 struct LagCellsLagrangeOnly {
   __device__ __forceinline__ void operator()(const RunView& v, int i, int j) const {
     Ctrl& C = *v.ctrl;
     unsigned long long dtb = ~0ull, pb = 0ull;
     if (i < v.ny && j < v.nx) {
-      LagCells<>{}(v, i, j);
+      LagCells<NB, 0, 0>{}(v, i, j);
       const long long c = (long long)i * v.nx + j, NP = v.npitch;
       const long long n0 = (long long)i * (v.nx + 1) + j;
       const long long nd[4] = {n0, n0 + 1, n0 + v.nx + 2, n0 + v.nx + 1};
@@ -2759,7 +2767,8 @@ __global__ void __launch_bounds__(kBX* kBY, 10) k_lag_nodes(RunView v) { split_n
 __global__ void __launch_bounds__(kBX* kBY, 8) k_lag_cells(RunView v) { plain_items(v, LagCells<>{}); }
 template <int NB, int PBV>
 __global__ void __launch_bounds__(kBX* kBY, 8) k_lag_cells_n(RunView v) { plain_items(v, LagCells<NB, PBV>{}); }
-__global__ void __launch_bounds__(kBX* kBY) k_lag_cells_lo(RunView v) { plain_items(v, LagCellsLagrangeOnly{}); }
+template <int NB>
+__global__ void __launch_bounds__(kBX* kBY) k_lag_cells_lo(RunView v) { plain_items(v, LagCellsLagrangeOnly<NB>{}); }
 __global__ void __launch_bounds__(kBX* kBY) k_next_positions(RunView v) { plain_items(v, NextPositions{}); }
 __global__ void __launch_bounds__(kBX* kBY) k_face_grad(RunView v, int sweep) { plain_items(v, FaceGrad{sweep}); }
 // Order 3: these wait on memory (eleven components in and out per cell);
@@ -3106,7 +3115,11 @@ int launch_cycle(const RunView& v, cudaStream_t s, const LaunchHook* hook,
   if (v.projection == 0) {
     // the Lagrange phase only: its cell kernel reduces the next dt, and the
     // new positions are carried to the next cycle after the loop test
-    H(3); k_lag_cells_lo<<<cg, blk, 0, s>>>(v); ++nk;
+    H(3);
+    if (v.nbmat == 1) k_lag_cells_lo<1><<<cg, blk, 0, s>>>(v);
+    else if (v.nbmat == 2) k_lag_cells_lo<2><<<cg, blk, 0, s>>>(v);
+    else k_lag_cells_lo<3><<<cg, blk, 0, s>>>(v);
+    ++nk;
     H(10); k_end<<<1, 1, 0, s>>>(v); ++nk;
     H(18); k_next_positions<<<ng, blk, 0, s>>>(v); ++nk;
     H(-1);
