@@ -1676,8 +1676,15 @@ struct SweepFaceT {
         // inputs below are finite and under 2^1000 (no sum or the factor 6
         // overflows).  The value itself is then not formed: 0 is stored
         // (the product's zero may differ in sign, which no later sum sees).
+        // Not for a face that a flux condition pairs with another face: the
+        // flux through a boundary face carries the value of the cell's
+        // opposite face, whatever that one's own velocity (bcf in
+        // SweepUpdateT; the top side's test takes every row there).
         constexpr unsigned long long kMod = 2023ull << 52;  // 2^1000
-        const bool still = v.pb == 0 && iszero(fnv) && is_finite(C.dt_n) && pos(h2) &&
+        const int fl = v.flux_bc;
+        const bool paired = dirx ? ((fl & kFluxLeft) && j == 1) || ((fl & kFluxRight) && j == v.nx - 1)
+                                 : ((fl & kFluxBottom) && i == 1) || (fl & kFluxTop);
+        const bool still = v.pb == 0 && !paired && iszero(fnv) && is_finite(C.dt_n) && pos(h2) &&
                            is_finite(h2);
         for (int k = 0; k < ncomp; ++k) {
           const double ys[3] = {v.o3y[k * FP + fidx - fst], v.o3y[k * FP + fidx],
