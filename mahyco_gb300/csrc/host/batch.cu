@@ -291,21 +291,15 @@ int get_plan(hydro_ctx* ctx, hydro_run* const* runs, int n, BatchPlan** out) {
 }
 
 int capture_graph(BatchPlan* p, int cycles) {
-  cudaStream_t s = p->ctx->stream;
   drop_graph(p);
-  cudaGraph_t g;
-  CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-  int nk = 0;
-  for (int k = 0; k < cycles; ++k) nk = launch_batch_cycle(p->L, s, nullptr, &p->ctx->fork);
-  cudaError_t e = cudaStreamEndCapture(s, &g);
-  if (e != cudaSuccess)
-    return fail(-40, std::string("batch graph capture: ") + cudaGetErrorString(e));
-  e = cudaGraphInstantiate(&p->graph, g, 0);
-  cudaGraphDestroy(g);
-  if (e != cudaSuccess)
-    return fail(-41, std::string("batch graph instantiate: ") + cudaGetErrorString(e));
+  if (int rc = capture_cycles(
+          p->ctx, cycles,
+          [&](cudaStream_t s, const CycleFork* f) {
+            return launch_batch_cycle(p->L, s, nullptr, f);
+          },
+          &p->graph, &p->kernels_per_cycle))
+    return rc;
   p->graph_cycles = cycles;
-  p->kernels_per_cycle = nk;
   return 0;
 }
 

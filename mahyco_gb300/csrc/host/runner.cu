@@ -182,11 +182,14 @@ int validate(const hydro_spec& s) {
   return 0;
 }
 
-void destroy_fork(CycleFork& f) {
+void destroy_fork(hydro_ctx* c) {
+  CycleFork& f = c->fork;
   for (auto& ev : f.ev)
     if (ev) cudaEventDestroy((cudaEvent_t)ev);
   if (f.side) cudaStreamDestroy((cudaStream_t)f.side);
   f = CycleFork{};
+  if (c->capture) cudaStreamDestroy(c->capture);
+  c->capture = nullptr;
 }
 
 }  // namespace
@@ -212,7 +215,8 @@ int hydro_ctx_create(int device, size_t budget, hydro_ctx** out) {
     return fail(-3, std::string("cudaStreamCreate: ") + cudaGetErrorString(e));
   }
   cudaStream_t side = nullptr;
-  e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
+  e = cudaStreamCreateWithFlags(&c->capture, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
   c->fork.side = side;
   for (auto& ev : c->fork.ev) {
     cudaEvent_t x = nullptr;
@@ -220,7 +224,7 @@ int hydro_ctx_create(int device, size_t budget, hydro_ctx** out) {
     ev = x;
   }
   if (e != cudaSuccess) {
-    destroy_fork(c->fork);
+    destroy_fork(c);
     cudaStreamDestroy(c->stream);
     delete c;
     return fail(-3, std::string("cudaStreamCreate: ") + cudaGetErrorString(e));
@@ -228,7 +232,7 @@ int hydro_ctx_create(int device, size_t budget, hydro_ctx** out) {
   // the pinned staging and host copy threads of hydro_run_fetch, set up
   // with the context rather than inside a run's first fetch
   if (int rc = create_fetch_stage(c->num_sms, &c->fetch)) {
-    destroy_fork(c->fork);
+    destroy_fork(c);
     cudaStreamDestroy(c->stream);
     delete c;
     return rc;
@@ -247,7 +251,7 @@ void hydro_ctx_destroy(hydro_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   destroy_fetch_stage(c->fetch);
   c->fetch = nullptr;
-  destroy_fork(c->fork);
+  destroy_fork(c);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
 }
@@ -435,6 +439,31 @@ int place_run(hydro_ctx* ctx, PreparedRun& pr, hydro_run** out, bool wait, bool 
   return 0;
 }
 
+int capture_cycles(hydro_ctx* ctx, int cycles,
+                   const std::function<int(cudaStream_t, const CycleFork*)>& cycle,
+                   cudaGraphExec_t* graph, int* kernels_per_cycle) {
+  std::lock_guard<std::mutex> lk(ctx->capture_mu);
+  cudaGraph_t g = nullptr;
+  CUDA_TRY(cudaStreamBeginCapture(ctx->capture, cudaStreamCaptureModeThreadLocal));
+  int nk = 0;
+  for (int k = 0; k < cycles; ++k) nk = cycle(ctx->capture, &ctx->fork);
+  // a launch refused during the capture would only be missing from the graph
+  const cudaError_t launch = cudaGetLastError();
+  cudaError_t e = cudaStreamEndCapture(ctx->capture, &g);
+  if (launch != cudaSuccess) e = launch;
+  const bool captured = e == cudaSuccess;
+  if (captured) e = cudaGraphInstantiate(graph, g, 0);
+  if (g) cudaGraphDestroy(g);
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // not left for a later call to report
+    *graph = nullptr;
+    return fail(captured ? -41 : -40, std::string(captured ? "graph instantiate: " : "graph capture: ") +
+                                          cudaGetErrorString(e));
+  }
+  *kernels_per_cycle = nk;
+  return 0;
+}
+
 }  // namespace hydro
 
 extern "C" {
@@ -466,22 +495,16 @@ namespace {
 
 // Captures `cycles` consecutive cycles of one run into a CUDA graph.
 int build_graph(hydro_run* r, int cycles) {
-  cudaStream_t s = r->ctx->stream;
   if (r->graph) {
     cudaGraphExecDestroy(r->graph);
     r->graph = nullptr;
   }
-  cudaGraph_t g;
-  CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-  int nk = 0;
-  for (int k = 0; k < cycles; ++k) nk = launch_cycle(r->v, s, nullptr, &r->ctx->fork);
-  cudaError_t e = cudaStreamEndCapture(s, &g);
-  if (e != cudaSuccess) return fail(-40, std::string("graph capture: ") + cudaGetErrorString(e));
-  e = cudaGraphInstantiate(&r->graph, g, 0);
-  cudaGraphDestroy(g);
-  if (e != cudaSuccess) return fail(-41, std::string("graph instantiate: ") + cudaGetErrorString(e));
+  if (int rc = capture_cycles(
+          r->ctx, cycles,
+          [&](cudaStream_t s, const CycleFork* f) { return launch_cycle(r->v, s, nullptr, f); },
+          &r->graph, &r->kernels_per_cycle))
+    return rc;
   r->graph_cycles = cycles;
-  r->kernels_per_cycle = nk;
   return 0;
 }
 

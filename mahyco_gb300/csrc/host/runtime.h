@@ -5,12 +5,15 @@
 
 #include <cuda_runtime.h>
 
+#include <functional>
 #include <mutex>
 #include <string>
 #include <vector>
 
 #include "../internal.h"
 #include "init.h"
+
+struct hydro_ctx;
 
 namespace hydro {
 
@@ -49,6 +52,15 @@ int place_run(hydro_ctx* ctx, PreparedRun& pr, hydro_run** out, bool wait,
               bool build_state = true);
 size_t run_arena_bytes(const hydro_spec& spec);
 
+// Captures `cycles` cycles, each queued by `cycle` (which returns its number
+// of kernels), into an executable graph.  The capture runs on a stream of the
+// context that nothing else uses: whatever other threads put on the context's
+// own stream meanwhile (a client fetching a served result while the worker
+// captures its batch) neither enters the graph nor ends the capture.
+int capture_cycles(::hydro_ctx* ctx, int cycles,
+                   const std::function<int(cudaStream_t, const CycleFork*)>& cycle,
+                   cudaGraphExec_t* graph, int* kernels_per_cycle);
+
 struct BatchPlan;
 struct ServeState;
 struct FetchStage;
@@ -66,7 +78,9 @@ struct hydro_ctx {
   size_t budget = 0;       // bytes of run state the context may hold (0: no cap)
   size_t used = 0;         // bytes of run state held
   cudaStream_t stream = nullptr;
+  cudaStream_t capture = nullptr;  // graphs are captured on it (capture_cycles)
   hydro::CycleFork fork;   // second stream and events of captured cycles
+  std::mutex capture_mu;   // one capture at a time: capture, fork
   std::mutex mu;
   hydro::BatchPlan* plan = nullptr;   // batch engine (lazily created)
   hydro::ServeState* serve = nullptr; // serving loop (lazily created)
