@@ -38,42 +38,54 @@ __device__ __forceinline__ void batch_items(const BatchArgs& b, const F& f, int 
 
 // Plain launches over the nodes, the boundary's apart: its nodes take a longer
 // path (fewer cells, the boundary conditions), and a warp with one of them
-// would run both.  The grid's first rows of blocks cover the four sides (the
-// corners with the bottom and the top), each from a warp of its own, since the
-// sides' conditions are different code; the others the inner nodes in tiles of
-// kNodeBX x kNodeBY.
+// would run both.  The grid's first columns of blocks cover the four sides
+// (the corners with the bottom and the top), each from a warp of its own, since
+// the sides' conditions are different code; the others the inner nodes in tiles
+// of kNodeBX x kNodeBY.  Columns, because a grid has at most 65535 rows of
+// blocks: the sides take none of them, so a mesh may have as many rows of cells
+// as the cells' own launches hold.
 constexpr int kNodeBX = 32, kNodeBY = 4;
 __host__ __device__ inline int side_warps(int n) { return (n + 31) / 32; }
-__host__ __device__ inline int perimeter_rows(const RunView& v, int gx) {
-  const int warps = 2 * side_warps(v.nx + 1) + 2 * side_warps(v.ny - 1);
-  return ((warps + kNodeBY - 1) / kNodeBY + gx - 1) / gx;
+inline int node_rows(int ny) { return (ny - 1 + kNodeBY - 1) / kNodeBY; }
+inline int perimeter_cols(int nx, int ny) {
+  const int warps = 2 * side_warps(nx + 1) + 2 * side_warps(ny - 1), gy = node_rows(ny);
+  return ((warps + kNodeBY - 1) / kNodeBY + gy - 1) / gy;
 }
-inline dim3 split_node_grid(const RunView& v) {
-  const int gx = (v.nx - 1 + kNodeBX - 1) / kNodeBX, gy = (v.ny - 1 + kNodeBY - 1) / kNodeBY;
-  return dim3(gx, gy + perimeter_rows(v, gx));
+inline dim3 split_node_grid(int nx, int ny) {
+  return dim3(perimeter_cols(nx, ny) + (nx - 1 + kNodeBX - 1) / kNodeBX, node_rows(ny));
+}
+// The node of thread (tx, ty) of block (bx, by); a side's node or an inner one.
+// cols: perimeter_cols (from the host: its division would lengthen every
+// thread's chain).
+struct SplitNode {
+  int i, j;
+  bool edge, inner;
+};
+__host__ __device__ inline SplitNode split_node_at(int nx, int ny, int cols, int bx, int by, int tx,
+                                                   int ty) {
+  if (bx >= cols) {
+    const int i = 1 + by * kNodeBY + ty, j = 1 + (bx - cols) * kNodeBX + tx;
+    return {i, j, false, i < ny && j < nx};
+  }
+  const int wx = side_warps(nx + 1), wy = side_warps(ny - 1);
+  int w = (by * cols + bx) * kNodeBY + ty;  // one row of threads: a warp
+  if (w < 2 * wx) {
+    const bool top = w >= wx;
+    const int j = (top ? w - wx : w) * 32 + tx;
+    return {top ? ny : 0, j, j <= nx, false};
+  }
+  w -= 2 * wx;
+  const bool right = w >= wy;
+  const int i = 1 + (right ? w - wy : w) * 32 + tx;
+  return {i, right ? nx : 0, w < 2 * wy && i < ny, false};
 }
 template <class F>
-__device__ __forceinline__ void split_node_items(const RunView& v, const F& f) {
+__device__ __forceinline__ void split_node_items(const RunView& v, int cols, const F& f) {
   if (!v.ctrl->active) return;
-  const int rows = perimeter_rows(v, gridDim.x), by = blockIdx.y;
-  if (by < rows) {
-    const int wx = side_warps(v.nx + 1), wy = side_warps(v.ny - 1);
-    int w = (by * gridDim.x + blockIdx.x) * kNodeBY + threadIdx.y;  // one row of threads: a warp
-    if (w < 2 * wx) {
-      const bool top = w >= wx;
-      const int j = (top ? w - wx : w) * 32 + threadIdx.x;
-      if (j <= v.nx) f.edge_node(v, top ? v.ny : 0, j);
-      return;
-    }
-    w -= 2 * wx;
-    if (w >= 2 * wy) return;
-    const bool right = w >= wy;
-    const int i = 1 + (right ? w - wy : w) * 32 + threadIdx.x;
-    if (i < v.ny) f.edge_node(v, i, right ? v.nx : 0);
-    return;
-  }
-  const int i = 1 + (by - rows) * kNodeBY + threadIdx.y, j = 1 + blockIdx.x * kNodeBX + threadIdx.x;
-  if (i < v.ny && j < v.nx) f.template node<true>(v, i, j);
+  const SplitNode n =
+      split_node_at(v.nx, v.ny, cols, blockIdx.x, blockIdx.y, threadIdx.x, threadIdx.y);
+  if (n.inner) f.template node<true>(v, n.i, n.j);
+  else if (n.edge) f.edge_node(v, n.i, n.j);
 }
 
 }  // namespace hydro

@@ -1,0 +1,43 @@
+// Every node of a mesh is visited once by the node launches' split grid, a
+// side's node as one and an inner one as one, and the grid is one that can be
+// launched.  Prints the number of meshes checked and of faulty ones.
+#include <cstdio>
+#include <vector>
+
+#include "kernels/items.cuh"
+
+namespace {
+bool check(int nx, int ny) {
+  const dim3 g = hydro::split_node_grid(nx, ny);
+  if (g.x < 1 || g.y < 1 || g.y > 65535u) return false;
+  const int cols = hydro::perimeter_cols(nx, ny);
+  std::vector<unsigned char> seen((size_t)(nx + 1) * (ny + 1), 0);
+  for (unsigned by = 0; by < g.y; ++by)
+    for (unsigned bx = 0; bx < g.x; ++bx)
+      for (int ty = 0; ty < hydro::kNodeBY; ++ty)
+        for (int tx = 0; tx < hydro::kNodeBX; ++tx) {
+          const hydro::SplitNode n = hydro::split_node_at(nx, ny, cols, (int)bx, (int)by, tx, ty);
+          if (!n.edge && !n.inner) continue;
+          if (n.i < 0 || n.i > ny || n.j < 0 || n.j > nx) return false;
+          const bool side = n.i == 0 || n.i == ny || n.j == 0 || n.j == nx;
+          if (n.edge != side || n.inner == side) return false;
+          if (seen[(size_t)n.i * (nx + 1) + n.j]++) return false;
+        }
+  for (unsigned char s : seen)
+    if (s != 1) return false;
+  return true;
+}
+}  // namespace
+
+int main() {
+  const int sizes[] = {2, 3, 4, 5, 6, 30, 31, 32, 33, 34, 63, 64, 65, 97, 128, 129, 301};
+  int n = 0, bad = 0;
+  for (int nx : sizes)
+    for (int ny : sizes) ++n, bad += !check(nx, ny);
+  // long thin meshes, to the most rows that the cells' and nodes' grids hold
+  for (int nx : {2, 8, 33, 34, 100})
+    for (int ny : {16383, 246700, 246800, 262139}) ++n, bad += !check(nx, ny);
+  for (int ny : {2, 5, 6}) ++n, bad += !check(1000003, ny);
+  std::printf("%d %d\n", n, bad);
+  return bad != 0;
+}
