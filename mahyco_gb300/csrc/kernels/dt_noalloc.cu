@@ -25,15 +25,15 @@
 
 namespace hydro {
 
-// Largest state accepted: 4096 * 256 = 1,048,576 cells.  A block takes kDtRows
-// x 31 cells per warp and at most kDtMaxBlocks blocks are launched, each with
-// one slot of the scratch (32 KiB).
+// Largest state accepted: 1,048,576 cells.  A warp takes units of R x 31 cells
+// (R rows, 1 to 8 by the mesh, DtGrid) and at most kDtMaxBlocks blocks are
+// launched, each with one slot of the scratch (32 KiB).
 constexpr long long kDtMaxCells = 1048576;
 constexpr int kDtMaxBlocks = 4096;
-constexpr int kDtRows = 8;      // rows of cells a warp takes at a time
+constexpr int kDtMaxRows = 8;   // most rows of cells of a unit
 constexpr int kDtCols = 31;     // columns of cells: 32 node columns a warp
-constexpr int kDtWarps = 8;     // warps of a block of the two-launch form
-constexpr int kDtOneWarps = 32; // largest single block
+constexpr int kDtMaxWarps = 16; // most warps of a block
+constexpr int kDtSms = 152;     // SMs of a GB300
 
 // One ordered-int partial minimum per block.  Every call overwrites the
 // slots of the blocks it launches before the final pass reads them, so
@@ -112,48 +112,57 @@ __device__ __forceinline__ float upper_float(unsigned hi, unsigned lo, bool& out
 // zero beside such a sound speed.  `all`: every cell forms it (cell sizes
 // for which the volumes' relative error has no such bound).
 //
-// A warp takes kDtRows x 31 cells: 32 node columns, one per lane, the right
+// The cells that form it go to a list of the block, from which all its threads
+// take them in turn: where the denominators tie (a mesh at rest, a uniform
+// flow) every cell is in it, and the FP64 pipe bounds the call as it does
+// without a filter.  So a block has as many cells as an SM's share of the
+// mesh (dt_grid).
+//
+// A warp takes R x 31 cells: 32 node columns, one per lane, the right
 // neighbour's speed by shuffle, the loads of all its rows issued before the
-// first use.  Calls back to back (GB300): 1024 x 1000 cells 315.4 -> 20.5 us,
-// 64 x 48 cells 20.0 -> 12.3 us (one launch instead of two, and the latency
-// of one exact candidate in place of every cell's).
+// first use.  Calls back to back (GB300), every cell's candidate formed ->
+// this: random fields 64 x 48 cells 18.5 -> 10.3 us, 200 x 200 30.7 -> 12.2,
+// 1024 x 1000 311 -> 16.4; at rest 20.3 -> 10.3, 30.8 -> 16.4, 326 -> 197.
 constexpr float kDtMargin = 1.0f - 1e-4f;
 
-template <int WARPS>
+template <int R>
 __device__ __forceinline__ unsigned long long block_min_candidate(
     int nx, int ny, double dx, double dy, const double* __restrict__ u,
     const double* __restrict__ v, const double* __restrict__ c, bool all) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int ncol = (nx + kDtCols - 1) / kDtCols, nrow = (ny + kDtRows - 1) / kDtRows;
+  const int ncol = (nx + kDtCols - 1) / kDtCols, nrow = (ny + R - 1) / R;
   const int units = ncol * nrow, nw = blockDim.x >> 5;
   const unsigned* uh = reinterpret_cast<const unsigned*>(u) + 1;
   const unsigned* vh = reinterpret_cast<const unsigned*>(v) + 1;
   const unsigned* ch = reinterpret_cast<const unsigned*>(c) + 1;
-  __shared__ float warp_max[WARPS];
+  __shared__ float warp_max[kDtMaxWarps];
+  // cells that form their candidate: (warp, row, lane) of this pass
+  __shared__ unsigned short list[kDtMaxWarps * R * 32];
+  __shared__ int listed;
   unsigned long long best = ~0ull;
   float seen = 0.0f;  // largest denominator of the block so far
   // the trip count is the block's, not the warp's (barriers inside)
   for (int base = blockIdx.x * nw; base < units; base += gridDim.x * nw) {
     const int unit = base + warp;
-    const int i0 = (unit / ncol) * kDtRows, j0 = (unit % ncol) * kDtCols, j = j0 + lane;
+    const int i0 = (unit / ncol) * R, j0 = (unit % ncol) * kDtCols, j = j0 + lane;
     const bool in = unit < units;
-    float s[kDtRows + 1], D[kDtRows];
-    unsigned hu[kDtRows + 1], hv[kDtRows + 1], hc[kDtRows];
+    float s[R + 1], D[R];
+    unsigned hu[R + 1], hv[R + 1], hc[R];
 #pragma unroll
-    for (int r = 0; r <= kDtRows; ++r) {
+    for (int r = 0; r <= R; ++r) {
       const bool node = in && j <= nx && i0 + r <= ny;
       const long long p = (long long)(i0 + r) * (nx + 1) + j;
       hu[r] = node ? __ldg(uh + 2 * p) : 0u;
       hv[r] = node ? __ldg(vh + 2 * p) : 0u;
     }
 #pragma unroll
-    for (int r = 0; r < kDtRows; ++r) {
+    for (int r = 0; r < R; ++r) {
       const bool cell = in && lane < kDtCols && j < nx && i0 + r < ny;
       hc[r] = cell ? __ldg(ch + 2 * ((long long)(i0 + r) * nx + j)) : 0u;
     }
     unsigned odd = 0;  // rows of nodes with a component of 2^61 or more
 #pragma unroll
-    for (int r = 0; r <= kDtRows; ++r) {
+    for (int r = 0; r <= R; ++r) {
       bool ou, ov;
       const float a = upper_float(hu[r], 897u, ou), b = upper_float(hv[r], 897u, ov);
       // out of range and not small
@@ -169,7 +178,7 @@ __device__ __forceinline__ unsigned long long block_min_candidate(
     unsigned take = 0;
     float top = 0.0f;
 #pragma unroll
-    for (int r = 0; r < kDtRows; ++r) {
+    for (int r = 0; r < R; ++r) {
       const float t = s[r] + s[r + 1];
       const float t1 = __shfl_down_sync(0xffffffffu, t, 1);
       const bool cell = in && lane < kDtCols && j < nx && i0 + r < ny;
@@ -182,24 +191,35 @@ __device__ __forceinline__ unsigned long long block_min_candidate(
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
     if (lane == 0) warp_max[warp] = top;
+    if (threadIdx.x == 0) listed = 0;
     __syncthreads();
     for (int w = 0; w < nw; ++w) seen = fmaxf(seen, warp_max[w]);
-    __syncthreads();
 #pragma unroll
-    for (int r = 0; r < kDtRows; ++r)
+    for (int r = 0; r < R; ++r) {
       if (D[r] > 0.0f && D[r] >= seen * kDtMargin) take |= 1u << r;
-    while (take) {
-      const int r = __ffs(take) - 1;
-      take &= take - 1;
-      const double d = exact_candidate(nx, i0 + r, j, dx, dy, u, v, c);
+      const unsigned m = __ballot_sync(0xffffffffu, (take >> r) & 1u);
+      if (m == 0) continue;
+      int at = 0;
+      if (lane == 0) at = atomicAdd(&listed, __popc(m));
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if ((take >> r) & 1u)
+        list[at + __popc(m & ((1u << lane) - 1u))] = (unsigned short)((warp * R + r) * 32 + lane);
+    }
+    __syncthreads();
+    const int n = listed;
+    for (int t = threadIdx.x; t < n; t += blockDim.x) {
+      const int e = list[t], w = base + (e >> 5) / R, r = (e >> 5) % R;
+      const double d = exact_candidate(nx, (w / ncol) * R + r, (w % ncol) * kDtCols + (e & 31), dx,
+                                       dy, u, v, c);
       if (!is_nan(d)) best = ord_bits(d) < best ? ord_bits(d) : best;
     }
+    __syncthreads();  // the list, its count and the maxima are written anew
   }
   for (int o = 16; o > 0; o >>= 1) {
     const unsigned long long t = __shfl_xor_sync(0xffffffffu, best, o);
     best = t < best ? t : best;
   }
-  __shared__ unsigned long long warp_min[WARPS];
+  __shared__ unsigned long long warp_min[kDtMaxWarps];
   if (lane == 0) warp_min[warp] = best;
   __syncthreads();
   for (int w = 0; w < nw; ++w) best = warp_min[w] < best ? warp_min[w] : best;
@@ -212,23 +232,35 @@ __device__ __forceinline__ double step_of(unsigned long long m, double dt_n) {
   return smin(red, 1.05 * dt_n);
 }
 
-__global__ void __launch_bounds__(kDtWarps * 32)
+template <int R>
+__global__ void __launch_bounds__(kDtMaxWarps * 32)
 k_dt_partial(int nx, int ny, double dx, double dy, const double* u,
              const double* v, const double* c, bool all, unsigned long long* scratch) {
   // the final pass may become resident now; it waits for this grid's end
   asm volatile("griddepcontrol.launch_dependents;");
-  const unsigned long long m = block_min_candidate<kDtWarps>(nx, ny, dx, dy, u, v, c, all);
+  const unsigned long long m = block_min_candidate<R>(nx, ny, dx, dy, u, v, c, all);
   if (threadIdx.x == 0) scratch[blockIdx.x] = m;
 }
 
-// Meshes of at most kDtOneWarps units (about 7900 cells): one block, one
-// launch, no scratch (the largest block the hardware takes; above it one
-// block would leave the other SMs idle).
-__global__ void __launch_bounds__(kDtOneWarps * 32)
-k_dt_one(int nx, int ny, double dx, double dy, const double* u, const double* v,
-         const double* c, bool all, double dt_n, double* dt_out) {
-  const unsigned long long m = block_min_candidate<kDtOneWarps>(nx, ny, dx, dy, u, v, c, all);
-  if (threadIdx.x == 0) *dt_out = step_of(m, dt_n);
+// Rows of a warp's units, and the launch: blocks of equal size, one per SM, or
+// k per SM where 16 warps of 8 rows do not hold an SM's share of the mesh.
+// The fewest rows with which one block per SM does: where all denominators tie
+// the time is that of the SM with the most cells (FP64 pipe), where one cell
+// decides it hardly depends on the rows.  (Blocks of 8 warps of 8 rows at every
+// size: at rest 129 us at 64 x 48 cells, 65 at 200 x 200, 227 at 1024 x 1000.)
+struct DtGrid {
+  int rows, warps, blocks;
+};
+DtGrid dt_grid(int nx, int ny) {
+  const long long ncol = (nx + kDtCols - 1) / kDtCols;
+  DtGrid g{1, 0, 0};
+  auto units = [&] { return ncol * ((ny + g.rows - 1) / g.rows); };
+  while (g.rows < kDtMaxRows && units() > kDtSms * kDtMaxWarps) g.rows *= 2;
+  const long long n = units(), most = kDtSms * kDtMaxWarps;
+  const long long slots = kDtSms * ((n + most - 1) / most);  // blocks of at most 16 warps
+  g.warps = (int)((n + slots - 1) / slots);
+  g.blocks = (int)std::min<long long>((n + g.warps - 1) / g.warps, kDtMaxBlocks);
+  return g;
 }
 
 constexpr int kDtBlock = 256;
@@ -306,30 +338,25 @@ extern "C" int hydro_vnr_dt_noalloc(int nx, int ny, double dx, double dy,
   const double w = std::fabs(dx * nx), h = std::fabs(dy * ny);
   auto plain = [](double x) { return x > 1e-70 && x < 1e70; };
   const bool all = !(dx > 0.0 && dy > 0.0 && plain(dx) && plain(dy) && plain(w) && plain(h));
-  const long long units = (long long)((nx + kDtCols - 1) / kDtCols) *
-                          ((ny + kDtRows - 1) / kDtRows);
-  if (units <= kDtOneWarps) {
-    k_dt_one<<<1, (unsigned)units * 32, 0, s>>>(nx, ny, dx, dy, d_u, d_v, d_c, all, dt_n,
-                                                d_dt_out);
-  } else {
-    const int nblocks = (int)std::min<long long>((units + kDtWarps - 1) / kDtWarps, kDtMaxBlocks);
-    k_dt_partial<<<nblocks, kDtWarps * 32, 0, s>>>(nx, ny, dx, dy, d_u, d_v, d_c, all, scratch);
-    // the final pass is launched ahead of the partial one's end
-    // (programmatic stream serialization)
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(1);
-    cfg.blockDim = dim3(kDtBlock);
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, k_dt_final, nblocks, dt_n,
-                           static_cast<const unsigned long long*>(scratch), d_dt_out);
-    if (e != cudaSuccess)
-      return fail(-6, std::string("hydro_vnr_dt_noalloc: launch: ") + cudaGetErrorString(e));
-  }
+  const DtGrid g = dt_grid(nx, ny);
+  auto partial = g.rows == 1 ? k_dt_partial<1> : g.rows == 2 ? k_dt_partial<2>
+               : g.rows == 4 ? k_dt_partial<4> : k_dt_partial<8>;
+  partial<<<g.blocks, g.warps * 32, 0, s>>>(nx, ny, dx, dy, d_u, d_v, d_c, all, scratch);
+  // the final pass is launched ahead of the partial one's end
+  // (programmatic stream serialization)
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(1);
+  cfg.blockDim = dim3(kDtBlock);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  e = cudaLaunchKernelEx(&cfg, k_dt_final, g.blocks, dt_n,
+                         static_cast<const unsigned long long*>(scratch), d_dt_out);
+  if (e != cudaSuccess)
+    return fail(-6, std::string("hydro_vnr_dt_noalloc: launch: ") + cudaGetErrorString(e));
   e = cudaGetLastError();
   if (e != cudaSuccess)
     return fail(-6, std::string("hydro_vnr_dt_noalloc: launch: ") + cudaGetErrorString(e));
