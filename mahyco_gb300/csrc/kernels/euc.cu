@@ -773,6 +773,7 @@ struct EucCells {
     }
   }
   __device__ __forceinline__ void operator()(const RunView& v, int i, int j) const {
+    const unsigned lanes = lanes_inside(i < v.ny && j < v.nx);
     if (i >= v.ny || j >= v.nx) return;
     const long long P = v.pitch, NP = v.npitch;
     const long long c = (long long)i * v.nx + j;
@@ -829,7 +830,7 @@ struct EucCells {
     single = single && pos(G.vol) && is_finite(G.vol) && nonneg(v.threshold);
     // the warp takes one of the two bodies: with both, its lanes would wait
     // for each other's (triple point 70 x 30: 45 us with one, 61 us with two)
-    if (__all_sync(__activemask(), single)) body<1>(v, c, nd, G, p);
+    if (__all_sync(lanes, single)) body<1>(v, c, nd, G, p);
     else body<3>(v, c, nd, G, 0);
   }
 };
@@ -861,7 +862,8 @@ struct EucFinal {
     if (pos(un1)) v.uco[P + c] = smax(un1, thr);
     else if (neg(un1)) v.uco[P + c] = smin(un1, -thr);
   }
-  static DV bool single(const RunView& v, long long c) {
+  // lanes: those of the warp that are inside the mesh, which all call this
+  static DV bool single(const RunView& v, long long c, unsigned lanes) {
     const long long P = v.pitch;
     const int nb = NB ? NB : v.nbmat;
     const double* U = v.UL + c;
@@ -882,7 +884,7 @@ struct EucFinal {
       }
     }
     // (a warp with a mixed cell takes the general path whole, not both)
-    if (!__all_sync(__activemask(), nonzero == 1)) return false;
+    if (!__all_sync(lanes, nonzero == 1)) return false;
     if (!(pos(vn) && is_finite(vn) && pos(um) && is_finite(um))) return false;
     const double q0 = U[3 * nb * P], q1 = U[(3 * nb + 1) * P];
     const double vol = ldg(v.evol, c);
@@ -919,11 +921,12 @@ struct EucFinal {
     return true;
   }
   __device__ __forceinline__ void operator()(const RunView& v, int i, int j) const {
+    const unsigned lanes = lanes_inside(i < v.ny && j < v.nx);
     if (i >= v.ny || j >= v.nx) return;
     Ctrl& C = *v.ctrl;
     const long long P = v.pitch;
     const long long c = (long long)i * v.nx + j;
-    if (single(v, c)) return;
+    if (single(v, c, lanes)) return;
     const int nb = NB ? NB : v.nbmat;
     const double thr = v.threshold;
     const double* U = v.UL + c;  // second sweep output

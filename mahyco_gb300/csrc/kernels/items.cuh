@@ -7,6 +7,11 @@
 
 namespace hydro {
 
+// The lanes of a warp whose item lies inside the mesh, for votes among them
+// after the others have left.  Called by whole warps (the plain and batched
+// launches have blocks of 128 threads that work on one tile).
+__device__ __forceinline__ unsigned lanes_inside(bool in) { return __ballot_sync(0xffffffffu, in); }
+
 // Batched launches: a persistent grid walks the tile table; every thread of
 // a block works on the same tile (the block reductions of some phases rely
 // on it).  The tile's run view is staged in shared memory by the whole

@@ -2394,14 +2394,15 @@ struct DualUpdate {
 // per value inside the general path, the shortcuts are if-converted into
 // FP64 instructions that run anyway.  Moving cells take it like those at
 // rest: FP64 instructions per cell of a moving flow 29 -> 9, 130 -> 74 us at
-// 1001 x 999 cells.
+// 1001 x 999 cells.  lanes: those of the warp that are inside the mesh, which
+// all call this.
 template <int NB>
 __device__ __forceinline__ bool final_single(const RunView& v, Ctrl& C, long long c, int nb,
                                              double thr, double vol, const double* vn,
                                              const double* Um, const double* Ue, double Uq,
                                              double c_in, double sarg_in, const double* spd,
                                              double cflsq, unsigned long long& dtb,
-                                             unsigned long long& pb) {
+                                             unsigned long long& pb, unsigned lanes) {
   constexpr unsigned long long kS = 0x8000000000000000ull;
   int p = -1, nonzero = 0;
   bool ok = nonneg(thr) && dlt(thr, 1.0);
@@ -2414,7 +2415,7 @@ __device__ __forceinline__ bool final_single(const RunView& v, Ctrl& C, long lon
     ok = ok && eos_of(v, m) == HYDRO_EOS_PERFECT_GAS && is_finite(gm1_of(v, m));
   }
   // (a warp with a mixed cell takes the general path whole, not both)
-  if (!__all_sync(__activemask(), ok && nonzero == 1)) return false;
+  if (!__all_sync(lanes, ok && nonzero == 1)) return false;
   // p's values by select over the unrolled materials (an index held in a
   // register would put the arrays in local memory)
   double vnp0 = 0., ump = 0., uep = 0.;
@@ -2472,7 +2473,7 @@ __device__ __forceinline__ bool final_single(const RunView& v, Ctrl& C, long lon
 template <int NB>
 __device__ __forceinline__ void final_cell(const RunView& v, Ctrl& C, int i,
                                            int j, unsigned long long& dtb,
-                                           unsigned long long& pb) {
+                                           unsigned long long& pb, unsigned lanes) {
   const long long P = v.pitch;
   const long long c = (long long)i * v.nx + j;
   const int nb = NB ? NB : v.nbmat;
@@ -2502,7 +2503,8 @@ __device__ __forceinline__ void final_cell(const RunView& v, Ctrl& C, int i,
     spd[3] = ld(v.speed, n0 + v.nx + 1);
     cflsq = ld(v.cflsq, c);
   }
-  if (final_single<NB>(v, C, c, nb, thr, vol, vn, Um, Ue, Uq, c_in, sarg_in, spd, cflsq, dtb, pb))
+  if (final_single<NB>(v, C, c, nb, thr, vol, vn, Um, Ue, Uq, c_in, sarg_in, spd, cflsq, dtb, pb,
+                       lanes))
     return;
   // every sum below starts from 0.0 in the reference: its first addition
   // 0.0 + x is plus_zero(x), on the integer pipe (materials 0 .. nb-1, nb >= 1)
@@ -2647,7 +2649,9 @@ struct Final {
   __device__ __forceinline__ void operator()(const RunView& v, int i, int j) const {
     Ctrl& C = *v.ctrl;
     unsigned long long dtb = ~0ull, pb = 0ull;
-    if (i < v.ny && j < v.nx) final_cell<NB>(v, C, i, j, dtb, pb);
+    const bool in = i < v.ny && j < v.nx;
+    const unsigned lanes = lanes_inside(in);
+    if (in) final_cell<NB>(v, C, i, j, dtb, pb, lanes);
     block_reduce_minmax(dtb, pb, &C);
   }
 };
