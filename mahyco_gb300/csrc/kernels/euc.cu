@@ -1070,7 +1070,7 @@ __device__ __forceinline__ void plain_items(const RunView& v, const F& f) {
 template <int NB>
 __global__ void __launch_bounds__(kBX* kBY, 8) ke_cell_pre(RunView v) { plain_items(v, EucCellPre<NB>{}); }
 template <int NB>
-__global__ void __launch_bounds__(kBX* kBY, 5) ke_nodes(RunView v, int cols) { split_node_items(v, cols, EucNodes<NB>{}); }
+__global__ void __launch_bounds__(kBX* kBY, 5) ke_nodes(RunView v, SplitGrid g) { split_node_items(v, g, EucNodes<NB>{}); }
 template <int NB>
 __global__ void __launch_bounds__(kBX* kBY, 8) ke_cells(RunView v) { plain_items(v, EucCells<NB>{}); }
 template <int NB>
@@ -1150,7 +1150,9 @@ static int launch_cycle_n(const RunView& v, cudaStream_t s, const LaunchHook* ho
   };
   H(0); ke_begin<<<1, 1, 0, s>>>(v); ++nk;
   H(12); ke_cell_pre<NB><<<cg, blk, 0, s>>>(v); ++nk;
-  H(13); ke_nodes<NB><<<split_node_grid(v.nx, v.ny), blk, 0, s>>>(v, perimeter_cols(v.nx, v.ny)); ++nk;
+  SplitGrid sg;
+  const dim3 sng = split_node_grid(v.nx, v.ny, &sg);
+  H(13); ke_nodes<NB><<<sng, blk, 0, s>>>(v, sg); ++nk;
   H(14); ke_cells<NB><<<cg, blk, 0, s>>>(v); ++nk;
   for (int sweep = 1; sweep <= 2; ++sweep) nk += launch_sweep(v, sweep, s, hook, nullptr);
   H(15); ke_final<NB><<<cg, blk, 0, s>>>(v); ++nk;

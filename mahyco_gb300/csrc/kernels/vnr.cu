@@ -2774,7 +2774,7 @@ __device__ __forceinline__ void plain_items(const RunView& v, const F& f) {
   f(v, blockIdx.y * kBY + threadIdx.y, blockIdx.x * kBX + threadIdx.x);
 }
 
-__global__ void __launch_bounds__(kBX* kBY, 10) k_lag_nodes(RunView v, int cols) { split_node_items(v, cols, LagNodes{}); }
+__global__ void __launch_bounds__(kBX* kBY, 10) k_lag_nodes(RunView v, SplitGrid g) { split_node_items(v, g, LagNodes{}); }
 __global__ void __launch_bounds__(kBX* kBY, 8) k_lag_cells(RunView v) { plain_items(v, LagCells<>{}); }
 template <int NB, int PBV>
 __global__ void __launch_bounds__(kBX* kBY, 8) k_lag_cells_n(RunView v) { plain_items(v, LagCells<NB, PBV>{}); }
@@ -3122,7 +3122,9 @@ int launch_cycle(const RunView& v, cudaStream_t s, const LaunchHook* hook,
     if (hook) (*hook)(kind);
   };
   H(0); k_begin<<<1, 1, 0, s>>>(v); ++nk;
-  H(2); k_lag_nodes<<<split_node_grid(v.nx, v.ny), blk, 0, s>>>(v, perimeter_cols(v.nx, v.ny)); ++nk;
+  SplitGrid sg;
+  const dim3 sng = split_node_grid(v.nx, v.ny, &sg);
+  H(2); k_lag_nodes<<<sng, blk, 0, s>>>(v, sg); ++nk;
   if (v.projection == 0) {
     // the Lagrange phase only: its cell kernel reduces the next dt, and the
     // new positions are carried to the next cycle after the loop test

@@ -8,15 +8,16 @@
 
 namespace {
 bool check(int nx, int ny) {
-  const dim3 g = hydro::split_node_grid(nx, ny);
+  hydro::SplitGrid sg;
+  const dim3 g = hydro::split_node_grid(nx, ny, &sg);
   if (g.x < 1 || g.y < 1 || g.y > 65535u) return false;
-  const int cols = hydro::perimeter_cols(nx, ny);
   std::vector<unsigned char> seen((size_t)(nx + 1) * (ny + 1), 0);
   for (unsigned by = 0; by < g.y; ++by)
     for (unsigned bx = 0; bx < g.x; ++bx)
       for (int ty = 0; ty < hydro::kNodeBY; ++ty)
         for (int tx = 0; tx < hydro::kNodeBX; ++tx) {
-          const hydro::SplitNode n = hydro::split_node_at(nx, ny, cols, (int)bx, (int)by, tx, ty);
+          const hydro::SplitNode n =
+              hydro::split_node_at(nx, ny, sg, (int)g.x, (int)bx, (int)by, tx, ty);
           if (!n.edge && !n.inner) continue;
           if (n.i < 0 || n.i > ny || n.j < 0 || n.j > nx) return false;
           const bool side = n.i == 0 || n.i == ny || n.j == 0 || n.j == nx;
