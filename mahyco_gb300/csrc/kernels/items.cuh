@@ -64,37 +64,38 @@ inline dim3 split_node_grid(int nx, int ny, SplitGrid* g) {
   else *g = {0, (blocks + gy - 1) / gy};
   return dim3(gx + g->cols, gy + g->rows);
 }
-// The node of thread (tx, ty) of block (bx, by) of a grid of gx columns; a side's
-// node or an inner one.
-struct SplitNode {
-  int i, j;
-  bool edge, inner;
-};
-__host__ __device__ inline SplitNode split_node_at(int nx, int ny, SplitGrid g, int gx, int bx,
-                                                   int by, int tx, int ty) {
-  if (by >= g.rows && bx >= g.cols) {
-    const int i = 1 + (by - g.rows) * kNodeBY + ty, j = 1 + (bx - g.cols) * kNodeBX + tx;
-    return {i, j, false, i < ny && j < nx};
+// What thread (tx, ty) of block (bx, by) of a grid of gx columns has: inner(i, j)
+// for an inner node, edge(i, j) for a side's.
+template <class Inner, class Edge>
+__host__ __device__ __forceinline__ void split_node(int nx, int ny, SplitGrid g, int gx, int bx,
+                                                    int by, int tx, int ty, const Inner& inner,
+                                                    const Edge& edge) {
+  if (by < g.rows || bx < g.cols) {
+    const int wx = side_warps(nx + 1), wy = side_warps(ny - 1);
+    int w = (by * (g.cols ? g.cols : gx) + bx) * kNodeBY + ty;  // one row of threads: a warp
+    if (w < 2 * wx) {
+      const bool top = w >= wx;
+      const int j = (top ? w - wx : w) * 32 + tx;
+      if (j <= nx) edge(top ? ny : 0, j);
+      return;
+    }
+    w -= 2 * wx;
+    if (w >= 2 * wy) return;
+    const bool right = w >= wy;
+    const int i = 1 + (right ? w - wy : w) * 32 + tx;
+    if (i < ny) edge(i, right ? nx : 0);
+    return;
   }
-  const int wx = side_warps(nx + 1), wy = side_warps(ny - 1);
-  int w = (by * (g.cols ? g.cols : gx) + bx) * kNodeBY + ty;  // one row of threads: a warp
-  if (w < 2 * wx) {
-    const bool top = w >= wx;
-    const int j = (top ? w - wx : w) * 32 + tx;
-    return {top ? ny : 0, j, j <= nx, false};
-  }
-  w -= 2 * wx;
-  const bool right = w >= wy;
-  const int i = 1 + (right ? w - wy : w) * 32 + tx;
-  return {i, right ? nx : 0, w < 2 * wy && i < ny, false};
+  const int i = 1 + (by - g.rows) * kNodeBY + ty, j = 1 + (bx - g.cols) * kNodeBX + tx;
+  if (i < ny && j < nx) inner(i, j);
 }
 template <class F>
 __device__ __forceinline__ void split_node_items(const RunView& v, SplitGrid g, const F& f) {
   if (!v.ctrl->active) return;
-  const SplitNode n = split_node_at(v.nx, v.ny, g, gridDim.x, blockIdx.x, blockIdx.y, threadIdx.x,
-                                    threadIdx.y);
-  if (n.inner) f.template node<true>(v, n.i, n.j);
-  else if (n.edge) f.edge_node(v, n.i, n.j);
+  split_node(
+      v.nx, v.ny, g, gridDim.x, blockIdx.x, blockIdx.y, threadIdx.x, threadIdx.y,
+      [&](int i, int j) { f.template node<true>(v, i, j); },
+      [&](int i, int j) { f.edge_node(v, i, j); });
 }
 
 }  // namespace hydro

@@ -12,21 +12,23 @@ bool check(int nx, int ny) {
   const dim3 g = hydro::split_node_grid(nx, ny, &sg);
   if (g.x < 1 || g.y < 1 || g.y > 65535u) return false;
   std::vector<unsigned char> seen((size_t)(nx + 1) * (ny + 1), 0);
+  bool ok = true;
   for (unsigned by = 0; by < g.y; ++by)
     for (unsigned bx = 0; bx < g.x; ++bx)
       for (int ty = 0; ty < hydro::kNodeBY; ++ty)
         for (int tx = 0; tx < hydro::kNodeBX; ++tx) {
-          const hydro::SplitNode n =
-              hydro::split_node_at(nx, ny, sg, (int)g.x, (int)bx, (int)by, tx, ty);
-          if (!n.edge && !n.inner) continue;
-          if (n.i < 0 || n.i > ny || n.j < 0 || n.j > nx) return false;
-          const bool side = n.i == 0 || n.i == ny || n.j == 0 || n.j == nx;
-          if (n.edge != side || n.inner == side) return false;
-          if (seen[(size_t)n.i * (nx + 1) + n.j]++) return false;
+          auto visit = [&](int i, int j, bool edge) {
+            const bool inside = i >= 0 && i <= ny && j >= 0 && j <= nx;
+            const bool side = i == 0 || i == ny || j == 0 || j == nx;
+            ok = ok && inside && side == edge && !seen[(size_t)i * (nx + 1) + j]++;
+          };
+          hydro::split_node(
+              nx, ny, sg, (int)g.x, (int)bx, (int)by, tx, ty,
+              [&](int i, int j) { visit(i, j, false); }, [&](int i, int j) { visit(i, j, true); });
         }
   for (unsigned char s : seen)
-    if (s != 1) return false;
-  return true;
+    ok = ok && s == 1;
+  return ok;
 }
 }  // namespace
 
