@@ -296,8 +296,8 @@ DV void bc_velocity(int bc, double V0, double V1, const double* Mp, const double
 //    other term made non-negative zero (x + (+-0) = x), its sums are +0, the
 //    determinant is Mp00 Mp11 - (+0), the inverse is diagonal up to zeros.
 // 1792 x 768 cells, 3 materials: 472 -> 322 us (five blocks per SM; four to
-// ten within 10 %); with the boundary's nodes in warps of their own 303 us,
-// and 70 x 30 cells 33 -> 22 us.
+// ten within 10 %); with the boundary's nodes in warps of their own and the
+// material count compiled in 296 us, and 70 x 30 cells 33 -> 22 us.
 template <int NB = 0>
 struct EucNodes {
   template <bool INNER>
@@ -531,7 +531,7 @@ struct EucNodes {
 //
 // The kernel is bound by the FP64 pipe (191 instructions per cell with all
 // materials and the full corner matrices in every cell: 734 us at 1792 x 768
-// cells and 3 materials, 475 us now; eight blocks per SM timed fastest of 3
+// cells and 3 materials, 427 us now; eight blocks per SM timed fastest of 3
 // to 8 there).  Three whole-cell reductions, each exact and one branch:
 //  - one material p (its fractions exactly 1, the others' fractions +0, their
 //    densities and corner pressures zeros): the others' forces are +0 (l * (a
@@ -846,7 +846,7 @@ struct EucCells {
 // vn_p', e_p = Ue_p / Um_p + dec, e = 0.0 + e_p, and the others' density +0
 // and energy 0.0 + dec.  A value that leaves these ranges (a negative or NaN
 // density or energy) returns false before any store.  One branch for the
-// cell: 35 -> 8 FP64 instructions, 119 -> 72 us at 1792 x 768 cells and 3
+// cell: 35 -> 8 FP64 instructions, 119 -> 64 us at 1792 x 768 cells and 3
 // materials.
 template <int NB = 0>
 struct EucFinal {

@@ -2394,8 +2394,8 @@ struct DualUpdate {
 // per value inside the general path, the shortcuts are if-converted into
 // FP64 instructions that run anyway.  Moving cells take it like those at
 // rest: FP64 instructions per cell of a moving flow 29 -> 9, 130 -> 74 us at
-// 1001 x 999 cells.  lanes: those of the warp that are inside the mesh, which
-// all call this.
+// 1001 x 999 cells (68 with the material count compiled in).  lanes: those of
+// the warp that are inside the mesh, which all call this.
 template <int NB>
 __device__ __forceinline__ bool final_single(const RunView& v, Ctrl& C, long long c, int nb,
                                              double thr, double vol, const double* vn,
@@ -2805,8 +2805,8 @@ __global__ void __launch_bounds__(kBX* kBY, 9) k_sweep_update_f(RunView v, int s
 // The usual component counts, known at compile time: 1001 x 999 cells moving 124
 // -> 113 us with PenteBorne (2 materials), 1792 x 768 cells at order 3 124 -> 102
 // us (3 materials, Eucclhyd).  Ten resident blocks with PenteBorne (at rest 80 us
-// at 2048 x 2048 cells against 84 with nine), eight without (102 us against 109
-// with six, 107 with nine).
+// at 2048 x 2048 cells against 84 with nine, before cells at rest left early: 45),
+// eight without (102 us against 109 with six, 107 with nine).
 template <int FACES, int NB, int NC>
 __global__ void __launch_bounds__(kBX* kBY, FACES ? 10 : 8) k_sweep_update_n(RunView v, int sweep) {
   plain_items(v, SweepUpdateT<FACES, NB, NC>{sweep});
@@ -2909,7 +2909,8 @@ __global__ void __launch_bounds__(128, 7) k_sweep_fused_y(RunView v, int sweep) 
   sweep_fused<false>(v, sweep);
 }
 __global__ void __launch_bounds__(kBX* kBY, 10) k_dual_grad(RunView v, int sweep) { plain_items(v, DualGrad{sweep}); }
-// ten resident blocks: where nodes are quiet the kernel waits on memory
+// twelve resident blocks: where nodes are quiet the kernel waits on memory (at
+// rest, 2048 x 2048 cells: 84 us, 91 at ten, 98 at eight; moving within 1 %)
 __global__ void __launch_bounds__(kBX* kBY, 12) k_dual_update(RunView v, int sweep) { plain_items(v, DualUpdate{sweep}); }
 template <int NB>
 __global__ void __launch_bounds__(kBX* kBY, 8) k_final(RunView v) { plain_items(v, Final<NB>{}); }
@@ -2977,7 +2978,8 @@ void launch_node_mass(const RunView& v, cudaStream_t s) {
   k_node_mass<<<node_grid(v), dim3(kBX, kBY), 0, s>>>(v);
 }
 
-// Kernel kinds of one cycle (for per-kernel timing).
+// Kernel kinds of one cycle (for per-kernel timing).  Kind 1 is kept for its
+// number only: k_begin resets the reductions.
 const char* const kKernelNames[kNumKernelKinds] = {
     "k_begin",      "k_reset_reductions", "k_lag_nodes", "k_lag_cells",
     "k_sweep_grad", "k_sweep_face",       "k_sweep_update", "k_dual_grad",
